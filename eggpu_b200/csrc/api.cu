@@ -226,16 +226,8 @@ void Plan::release() {
     cg = nullptr;
     cond = 0;
     cg_failed = false;
-    d_chunks.release();
-    d_graphs.release();
-    d_states.release();
-    d_ndang.release();
-    d_ctl.release();
-    d_acc.release();
-    d_span_acc.release();
-    d_span_cnt.release();
-    d_span_list.release();
-    ngraphs = nchunks = grid = any_weighted = max_n = nspans = nacc = 0;
+    for (DevBuf* b : {&d_units, &d_cta_unit, &d_row_tiles, &d_graphs, &d_states, &d_ndang, &d_ctl, &d_acc}) b->release();
+    ngraphs = grid = row_grid = nrow_tiles = max_rows = max_n = nacc = 0;
 }
 
 void Plan::release_on(cudaStream_t s) {
@@ -245,9 +237,9 @@ void Plan::release_on(cudaStream_t s) {
     cg = nullptr;
     cond = 0;
     cg_failed = false;
-    for (DevBuf* b : {&d_chunks, &d_graphs, &d_states, &d_ndang, &d_ctl, &d_acc, &d_span_acc, &d_span_cnt, &d_span_list})
+    for (DevBuf* b : {&d_units, &d_cta_unit, &d_row_tiles, &d_graphs, &d_states, &d_ndang, &d_ctl, &d_acc})
         b->release_on(s);
-    ngraphs = nchunks = grid = any_weighted = max_n = nspans = nacc = 0;
+    ngraphs = grid = row_grid = nrow_tiles = max_rows = max_n = nacc = 0;
 }
 
 int check_device(const egpr_graph* g) {
@@ -315,7 +307,7 @@ static int read_states(Plan& plan, int32_t idx, cudaStream_t s, SolveOut* o) {
     return EGPR_SUCC;
 }
 
-// The state of a graph's last single-vector solve (binned or tile sweep).
+// The state of a graph's last single-vector solve (binned or blocked sweep).
 static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
     if (!g->bins) return read_states(g->plan, 0, s, o);
     return bins_read_state(g, s, &o->iterations, &o->converged, &o->residual, &o->launches, &o->error);
@@ -512,13 +504,13 @@ static uint64_t bits_of(double x) {
 }  // namespace egpr
 
 int64_t egpr_graph::device_bytes() const {
-    return (int64_t)(in_row.bytes + in_col.bytes + in_w.bytes + outw.bytes + dangling01.bytes +
-                     sw_row.bytes + sw_col.bytes + sw_w.bytes + tile_bits.bytes + tile_row.bytes +
-                     hub_ids.bytes + hub_slot.bytes + hubz.bytes + hubz64.bytes + plan.d_acc.bytes + plan.d_span_acc.bytes + plan.d_span_cnt.bytes +
-                     plan.d_span_list.bytes +
-                     scale.bytes + tele.bytes + x0.bytes + x1.bytes + z0.bytes + z1.bytes + out.bytes + z64.bytes +
-                     plan.d_chunks.bytes + plan.d_graphs.bytes + plan.d_states.bytes + plan.d_ndang.bytes +
-                     plan.d_ctl.bytes) + (bins ? bins->device_bytes() : 0);
+    int64_t b = 0;
+    for (const egpr::DevBuf* d : {&in_row, &in_col, &in_w, &outw, &dangling01, &rank, &idx, &sw_w, &tile_bits, &tile_pair,
+                            &pair_row, &row_step, &steps, &row_tile, &pairs, &scale, &tele, &x0, &x1, &z0, &out, &z64, &plan.d_units,
+                            &plan.d_cta_unit, &plan.d_row_tiles, &plan.d_graphs, &plan.d_states, &plan.d_ndang,
+                            &plan.d_ctl, &plan.d_acc})
+        b += (int64_t)d->bytes;
+    return b + (bins ? bins->device_bytes() : 0);
 }
 
 using namespace egpr;
@@ -534,10 +526,9 @@ static void destroy_graph_object(egpr_graph* g) {
     delete g->bins;
     g->bins = nullptr;
     g->plan.release();
-    for (DevBuf* b : {&g->in_row, &g->in_col, &g->in_w, &g->outw, &g->dangling01, &g->sw_row,
-                      &g->sw_col, &g->sw_w, &g->tile_bits, &g->tile_row,
-                      &g->hub_ids, &g->hub_slot, &g->hubz, &g->hubz64, &g->scale, &g->tele, &g->seed_ids,
-                      &g->x0, &g->x1, &g->z0, &g->z1, &g->out, &g->z64})
+    for (DevBuf* b : {&g->in_row, &g->in_col, &g->in_w, &g->outw, &g->dangling01, &g->rank, &g->idx, &g->sw_w,
+                      &g->tile_bits, &g->tile_pair, &g->pair_row, &g->row_step, &g->steps, &g->row_tile, &g->pairs, &g->scale, &g->tele,
+                      &g->seed_ids, &g->x0, &g->x1, &g->z0, &g->out, &g->z64})
         b->release();
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
@@ -687,12 +678,9 @@ int rebuild_sweep(egpr_graph* g) {
         (rc = cuda_ok(cudaStreamSynchronize(s), "tuning")))
         return rc;
     drop_multi_plans_with(g);  // they hold copies of the graph's chunk table
-    if ((rc = build_sweep_layout(g, sweep_resident_warps(), nullptr, s))) return rc;
+    if ((rc = rebuild_sweep_layout(g, s))) return rc;
     egpr_graph* self = g;
-    if ((rc = plan_build(g->plan, &self, 1, s))) return rc;
-    const size_t nf = ((size_t)g->n + 8) * sizeof(float);
-    plan_set_l2_window(g->plan, g->z0.p, 2 * nf);
-    return EGPR_SUCC;
+    return plan_build(g->plan, &self, 1, s);
 }
 
 // Device time of one sweep of the graph's current layout: fixed-count solves
@@ -813,17 +801,10 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
             return rc;
         }
     }
-    // Row arrays are read by 16-byte bulk copies that may run up to 3 elements past n.
-    const size_t nf = ((size_t)n + 8) * sizeof(float), nd = (size_t)n * sizeof(double);
-    if ((rc = g->scale.alloc(nf)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
-        (rc = g->z0.alloc(2 * nf)) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nd + sizeof(double))) ||
-        (rc = g->hubz.alloc(2 * (size_t)hub_stride(g->nhub) * sizeof(float))) ||
-        (rc = g->hubz64.alloc(((size_t)g->nhub + 1) * sizeof(double))) ||
-        // zero slots: hubz[.][nhub] and z64[n] are read by placeholder entries
-        (rc = (cudaMemsetAsync(g->hubz.p, 0, g->hubz.bytes, g->own_stream) == cudaSuccess &&
-               cudaMemsetAsync(g->z64.p, 0, g->z64.bytes, g->own_stream) == cudaSuccess)
-                  ? EGPR_SUCC
-                  : set_cuda_error(cudaGetLastError(), "memset"))) {
+    const size_t nf = (size_t)n * sizeof(float), nd = (size_t)n * sizeof(double);
+    const size_t nz = (size_t)z_stride(g->nsrc);  // by source rank, whole 16-byte units
+    if ((rc = g->scale.alloc(2 * nf)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
+        (rc = g->z0.alloc(2 * nz * sizeof(float))) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nz * sizeof(double)))) {
         destroy_graph_object(g);
         return rc;
     }
@@ -832,7 +813,6 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
         destroy_graph_object(g);
         return rc;
     }
-    plan_set_l2_window(g->plan, g->z0.p, 2 * nf);
     *out = g;
     return EGPR_SUCC;
 }

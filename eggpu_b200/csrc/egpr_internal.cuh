@@ -13,72 +13,87 @@
 namespace egpr {
 
 // ---------------------------------------------------------------------------
-// Work decomposition of the single-vector sweep.
+// Layout of the single-vector sweep.
 //
-// The sweep reads the inbound CSR with one placeholder entry in every empty
-// row, in warp tiles of kTileItems entries.  Runs of tiles form chunks, cut at
-// equal cost (entries plus a weight per row), the unit of the persistent work
-// queue.  A row cut by a chunk boundary is a "span": each chunk it touches
-// adds its piece, and the last of them to arrive finishes the row (no
-// waiting; the pieces are exact fixed point, so the order does not matter).
+// A random 4-byte read that misses L1 costs an SM one 32-byte sector from L2,
+// and an SM receives about one sector per clock (measured on B200: 289 G such
+// reads/s over all SMs, from any vector that fits L2), while shared memory
+// serves 11 random reads per clock.  So no carried value is gathered from
+// global memory:
+//   * sources (vertices with out-edges) are ranked by out-degree and cut into
+//     blocks of kBlockSrc; the carried values z are stored in rank order, so a
+//     block's values are one contiguous piece that a CTA stages in shared memory;
+//   * the inbound entries are ordered by (block, destination); each is a 16-bit
+//     index into its block;
+//   * phase 1 (k_gather) sums every run of entries of one (block, row) into a
+//     "pair", written in order; phase 2 (k_rows) adds the pairs of each row
+//     from all blocks in shared memory and finishes the row.
+// Ranking by degree packs the entries into few runs: R-MAT scale 22 has 0.17
+// pairs per entry (0.30 with blocks in vertex order).
+//
+// A graph with too many (block, row tile) cells for the list of steps (about
+// 3 * 10^8 vertices and more) is laid out as one block of any size whose values are
+// read from global memory (32-bit ranks instead of 16-bit indices).
 // ---------------------------------------------------------------------------
 constexpr int kThreads = 256;  // threads of the preparation and helper kernels
 
-// Chunk flags.
+// Span flags of the batched solve's chunks (spmm.cu).
 constexpr int32_t kHasHead = 1;    // the chunk's first row began in an earlier chunk
 constexpr int32_t kHasTail = 2;    // the chunk's last row continues into a later chunk
 constexpr int32_t kInterior = 4;   // the chunk lies inside one row (head and tail are that row)
 
-struct Chunk {
-    int32_t tile_begin;  // first warp tile of the chunk
-    int32_t tile_end;    // one past its last warp tile
-    int32_t graph;       // slot in the plan's graph table
-    int32_t flags;
-    int32_t head_ta;     // global chunk id where the head row's span starts
-    int32_t tail_tb;     // global chunk id where the tail row's span ends
-    int32_t tail_row;    // vertex id of the tail row (span rows are finalised by row id)
-    int32_t pad2;        // sweep chunk: chunks of its tail row's span
-    int32_t nnz_begin;   // entries [nnz_begin, nnz_end) belong to the chunk
-    int32_t nnz_end;
-    int32_t row_end;     // sweep chunk: rows before row_end are finished by the chunk
-    int32_t pad;         // sweep chunk: chunks of its head row's span (estimated cost while preparing)
-};
-
-// The sweep's warp tiles: kTileItems entries, lane l owning entries 8l..8l+7.
+// Sources per block: FP64 values of one block (176 KB, the correction sweep) and
+// a tile of row sums per warp (48 KB) fill the shared memory of an SM.
+constexpr int32_t kBlockSrc = 22528;
+constexpr int kBlockBits = 15;     // bits of an index inside a block (kBlockSrc itself is the zero slot)
+// Warp tiles of kTileItems entries, lane l owning entries 8l..8l+7.  A block's
+// entries are padded to whole tiles with zero-slot entries.  A warp walks chunks of
+// 2^chunk_shift tiles (counted from the block's first one); a run never leaves its
+// chunk (a longer one becomes several pairs), so chunks are independent.
 constexpr int kLaneItems = 8;
 constexpr int kTileItems = 32 * kLaneItems;
-// Per-tile words of the tile table: 8 words of row-end marks (one byte per
-// lane), then 8 words with, per lane, the marks of the lanes below it.
+// Per tile and lane one 16-bit word: the lane's run-end marks (low byte) and the
+// number of marks in the lanes below it (high byte); 64 bytes per tile.
 constexpr int kTileWords = 16;
-// Hub cache: the carried values of the (up to kHubCap - 32) sources with the
-// largest out-degree are kept in shared memory by the sweep; inbound entries
-// from a hub store -(slot + 1) instead of the source id.  Slot nhub holds 0 and
-// is read by the placeholder entry of every row without entries.
-constexpr int kHubCap = 49152;      // largest hub cache (values) a sweep CTA stages
+// Row tiles of phase 2: runs of whole 32-row groups of about equal cost, at most
+// kMaxTileRows rows, summed in one CTA's shared memory.
+constexpr int kRowGroup = 32;
+constexpr int32_t kMinTileRows = 256;    // wanted at least (fewer where rows are heavy)
+constexpr int32_t kMaxTileRows = 12288;  // 96 KB of FP32 sweep sums (two CTAs per SM), 192 KB of FP64 ones
+constexpr int kRowTilesPerSm = 2;        // CTAs of phase 2 that an SM holds
+constexpr int kStepPairs = 128;          // pairs of one block that a warp adds at a time
 
 // Per-graph device view used by the sweep kernels.
 struct GraphDev {
-    const int32_t* cols;        // sweep entries: hub-encoded sources, a placeholder in every empty row
-    const float* w;             // their weights, NULL = unit weights
-    const uint32_t* tile_bits;  // per warp tile: kTileWords words (row-end marks, per-lane mark offsets)
-    const int32_t* tile_row;    // per warp tile: the row its first mark ends
+    const uint16_t* idx;        // per padded entry: index of its source in the block (kBlockSrc: none)
+    const int32_t* idx32;       // one-block layout without staging: rank of the source (-1: none); else NULL
+    const float* w;             // weights of the padded entries, NULL = unit weights
+    const uint32_t* tile_bits;  // per tile: kTileWords words (run-end marks, per-lane mark offsets)
+    const int32_t* tile_pair;   // per tile: its first pair (ntiles + 1)
+    const uint16_t* pair_row;   // per pair: its row in its row tile
+    const int32_t* row_step;    // first step of each row tile (one more than there are row tiles)
+    const int2* steps;          // (first pair, pairs): up to kStepPairs pairs of one block and row tile
+    const int32_t* row_tile;    // first row of each row tile (one more than there are row tiles)
+    void* pairs;                // per pair: its sum (FP32, or FP64 in the correction sweep)
     const double* outw;      // n, FP64 out-weight sums
-    const float* scale;      // n, alpha/outw (FP32) or -1 for dangling vertices
+    const int32_t* rank;     // n, rank of each source, -1 for a vertex without out-edges
+    const float2* rowd;      // n, what finishing a row needs: alpha/outw (FP32, -1 for dangling), rank (int32 bits)
     const float* tele;       // n, personalisation (NULL = uniform)
     float* x[2];             // ranks, double-buffered
-    float* z[2];             // x * scale: the value each out-edge carries
+    float* z[2];             // by source rank: x * alpha/outw, the value each out-edge carries
     double* out;             // n, FP64 result
-    double* z64;             // n, FP64 carried values for the correction sweep
-    const int32_t* hub_ids;  // nhub source ids of the hub slots
-    const int32_t* hub_slot; // n, slot of each vertex or -1
-    float* hubz[2];          // nhub carried values of the hubs, double-buffered with z
-    double* hubz64;          // nhub + 1: the hubs' FP64 carried values for the correction sweep (slot nhub = 0)
-    int32_t nhub;
+    double* z64;             // by source rank: FP64 carried values for the correction sweep
     int32_t n;
-    int32_t chunk_begin;     // this graph's global chunk id range
-    int32_t chunk_end;
-    int32_t span_begin;      // this graph's entries of the span list (span start stages)
-    int32_t span_end;
+    int32_t nsrc;            // ranked sources
+    int32_t nblocks;
+    int32_t chunk_shift;
+};
+
+// A CTA's piece of phase 1: tiles [tile0, tile1) of one block of one graph.
+struct GatherUnit {
+    int32_t graph;
+    int32_t block;
+    int32_t tile0, tile1;
 };
 
 struct GraphState {
@@ -95,7 +110,7 @@ struct GraphState {
     int32_t max_iter;
     int32_t done;
     int32_t converged;
-    uint32_t arrive;   // chunk arrivals in the running launch
+    float fx_unit;     // phase 2 adds in units of 1 / fx_unit (a power of two)
     int32_t personalised;  // teleport from GraphDev::tele instead of 1/n
 };
 
@@ -111,25 +126,22 @@ struct Ctl {
 constexpr int kAccWords = 8;  // words per accumulator slot (6 used; 64-byte slots)
 
 struct SweepParams {
-    const Chunk* chunks;     // in queue order (costliest chunks of a graph first)
-    int32_t nchunks;
-    int32_t mode;            // 0 = FP32 sweep, 1 = FP64 correction sweep
+    const GatherUnit* units;
+    const int32_t* cta_unit;       // per phase 1 CTA: its first unit (grid + 1)
+    const int2* row_tiles;         // (graph, row tile), in row order
+    int32_t nrow_tiles;
+    int32_t max_rows;              // of a row tile in the plan: the size of a CTA's row sums
     const GraphDev* graphs;
     GraphState* states;
     // FP64 sums are accumulated as two's-complement fixed point (2 words: units
     // of 2^-32 and of 2^-64) with integer atomics, so their order does not
     // change the result.
     unsigned long long* acc;       // kAccWords per slot: err, dangling, rank sums
-    unsigned long long* span_acc;  // 2 per chunk (span start chunk): the cut row's sum
-    uint32_t* span_cnt;            // per chunk (span start chunk): pieces added so far
-    const int32_t* span_list;  // span start stages
-    int32_t nspans;
-    int32_t acc_sub;           // accumulator slots per graph
+    int32_t acc_sub;               // accumulator slots per graph
     Ctl* ctl;
     cudaGraphConditionalHandle cond;
     int32_t use_cond;
     int32_t ngraphs;
-    int32_t hub_count;       // hub slots staged in shared memory (0: hubs read from global memory)
 };
 
 // ---- device buffers --------------------------------------------------------
@@ -152,24 +164,17 @@ struct DevBuf {
 // ---- the work plan over one or more prepared graphs -------------------------
 struct Plan {
     int32_t ngraphs = 0;
-    int32_t nchunks = 0;
-    int32_t grid = 0;        // CTAs of a sweep
-    int32_t any_weighted = 0;
-    int32_t hub_count = 0;   // hubs of the plan's graph (one-graph plans)
+    int32_t grid = 0;        // CTAs of phase 1
+    int32_t row_grid = 0;    // CTAs of phase 2
+    int32_t nrow_tiles = 0;
+    int32_t max_rows = 0;    // of a row tile
     int32_t max_n = 0;
-    DevBuf d_chunks, d_graphs, d_states, d_ndang, d_ctl, d_span_list, d_acc, d_span_acc, d_span_cnt;
-    std::vector<Chunk> h_chunks;      // a graph's own chunk table (local ids)
-    std::vector<int32_t> h_spans;     // a graph's span start chunks (local ids)
-    std::vector<Chunk> h_chunks_all;  // the plan's table (global ids)
-    int32_t nspans = 0;
+    DevBuf d_units, d_cta_unit, d_row_tiles, d_graphs, d_states, d_ndang, d_ctl, d_acc;
     int32_t nacc = 0;                 // accumulator slots
     cudaGraph_t cg = nullptr;
     cudaGraphExec_t cg_exec = nullptr;
     cudaGraphConditionalHandle cond = 0;
     bool cg_failed = false;
-    void* l2_base = nullptr;  // persisting L2 window over the gathered vectors
-    size_t l2_bytes = 0;
-    float l2_hit_ratio = 0.f;
     ~Plan();
     void release();
     void release_on(cudaStream_t s);  // buffers used by stream s only: freed in its order
@@ -259,19 +264,24 @@ struct egpr_graph {
     int32_t host_inputs_locked = 0;      // host input arrays that were page-locked already
     int32_t host_inputs_staged = 0;      // host input arrays copied through the staging pool
     // prepared graph
-    egpr::DevBuf in_row, in_col, in_w, outw, dangling01, hub_ids, hub_slot, hubz, hubz64;
+    egpr::DevBuf in_row, in_col, in_w, outw, dangling01, rank;
     // the sweep's layout (see build_sweep_layout)
-    egpr::DevBuf sw_row, sw_col, sw_w, tile_bits, tile_row;
-    int64_t sw_nnz = 0;
-    int32_t ntiles = 0;
-    int32_t nhub = 0;
+    egpr::DevBuf idx, sw_w, tile_bits, tile_pair, pair_row, row_step, steps, row_tile, pairs;
+    int32_t nsrc = 0;              // ranked sources
+    int32_t nblocks = 0;
+    int32_t chunk_shift = 0;       // log2 of the tiles per chunk
+    int32_t global_block = 0;      // one block, values read from global memory (idx holds 32-bit ranks)
+    int32_t max_tile_rows = 0;     // rows of the largest row tile, rounded up
+    std::vector<int32_t> h_block_tile;  // first tile of each block (nblocks + 1)
+    std::vector<int32_t> h_block_pair;  // first pair of each block (nblocks + 1)
+    int32_t nrow_tiles = 0;
     // layout parameters (egpr_tuning); defaults from the environment
-    int32_t tune_cpw = 8;           // sweep: work-queue chunks per resident warp
-    int32_t tune_rc = 4;            // sweep: cost of finishing a row, in entries
+    int32_t tune_cpw = 8;           // sweep: sets the row tile size (row tiles per resident warp)
+    int32_t tune_rc = 4;            // sweep: cost of a pair, in entries, when phase 1 is cut into CTA shares
     int32_t tune_spmm_chunk = 1024; // batched solve: entries per work unit
     int32_t tuning_recorded = 0;    // the layout came from the persisted tuner choices
     // solve workspace
-    egpr::DevBuf scale, tele, x0, x1, z0, z1, out, z64;
+    egpr::DevBuf scale, tele, x0, x1, z0, out, z64;
     egpr::DevBuf seed_ids;         // seed set of a single-vector PPR solve
     egpr::Plan plan;               // single-graph plan
     egpr::SpmmWork* spmm = nullptr; // batched personalised PageRank workspace
@@ -304,7 +314,9 @@ double wall_seconds();
 
 // Preparation (prep.cu).
 int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const double* W);
-int build_sweep_layout(egpr_graph* g, int32_t resident_warps, const uint32_t* sorted_dst, cudaStream_t s);
+int rebuild_sweep_layout(egpr_graph* g, cudaStream_t s);  // for the graph's current layout parameters
+// Destination of every inbound entry, in entry order (row offsets expanded).
+void expand_rows(const int32_t* row, int32_t n, int32_t* dst, cudaStream_t s);
 int default_chunks_per_warp();  // EGPR_CHUNKS_PER_WARP, else 8
 int default_row_cost();         // EGPR_ROW_COST, else 4
 int32_t default_spmm_chunk();   // EGPR_SPMM_CHUNK, else 1024
@@ -329,10 +341,9 @@ int bins_read_state(egpr_graph* g, cudaStream_t s, int32_t* iterations, int32_t*
 int sweep_grid();
 int sweep_resident_warps();
 int work_grid(int64_t entries, int full);  // CTAs of a launch over that many entries
-int32_t hub_stride(int32_t nhub);  // floats per parity of the hub copy (zero slot included)
+int64_t z_stride(int32_t nsrc);    // values per parity of z (whole 16-byte units past the last block)
 int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_t stream);
 int plan_capture_loop(Plan& plan, cudaStream_t stream);
-void plan_set_l2_window(Plan& plan, void* base, size_t bytes);
 GraphDev graph_dev_view(const egpr_graph* g);
 int launch_init(Plan& plan, double alpha, int32_t max_iter, double tol, bool personalised,
                 cudaStream_t stream);

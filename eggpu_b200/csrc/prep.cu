@@ -238,6 +238,19 @@ __device__ __forceinline__ int lsb_exponent(double w) {
     return e + __ffsll((long long)m) - 1;
 }
 
+// Ranking key of a source with c valid out-edges: descending classes of an
+// eighth of an octave, 255 for none.  Classes instead of exact degrees: one
+// 8-bit sort pass ranks the vertices, and inside a class the order stays that
+// of the vertices, so neighbouring rows of similar degree have neighbouring
+// ranks and their carried values are written in few sectors.
+constexpr uint32_t kNoRank = 255u;
+__device__ __forceinline__ uint32_t rank_class(int32_t c) {
+    if (c <= 0) return kNoRank;
+    const int e = 31 - __clz(c);                                       // octave
+    const int f = e >= 3 ? (c >> (e - 3)) & 7 : (c << (3 - e)) & 7;    // eighth of it
+    return (uint32_t)(254 - (8 * e + f));                              // 8 * 30 + 7 at most
+}
+
 // FP64 out-weight sums, one warp per source, bit-identical to the sequential
 // sum in entry order (pagerank.cu:301-316) without summing sequentially.
 // Sanitised weights are >= 0; let 2^q be the lowest set bit among a row's
@@ -278,7 +291,7 @@ __device__ __forceinline__ void out_weight_row(const int32_t* __restrict__ E, co
 // is provably exact (see above); otherwise the source is listed for the
 // sequential kernel.
 __device__ __forceinline__ void out_weight_store(int64_t u, double s, int32_t c, int q, double* __restrict__ outw,
-                                                 uint32_t* __restrict__ hub_key, uint32_t* __restrict__ hub_val,
+                                                 uint32_t* __restrict__ rank_key, uint32_t* __restrict__ rank_val,
                                                  int32_t* __restrict__ serial_rows,
                                                  uint32_t* __restrict__ serial_count) {
     bool exact;
@@ -287,9 +300,8 @@ __device__ __forceinline__ void out_weight_store(int64_t u, double s, int32_t c,
     else exact = s < ldexp(1.0, q + 52);
     if (exact) outw[u] = s;
     else serial_rows[atomicAdd(serial_count, 1u)] = (int32_t)u;
-    // hub ranking: descending out-degree, ascending id (stable sort of ~count)
-    hub_key[u] = ~(uint32_t)c;
-    hub_val[u] = (uint32_t)u;
+    rank_key[u] = rank_class(c);
+    rank_val[u] = (uint32_t)u;
 }
 
 constexpr int32_t kOutWeightShort = 64;  // sources with more entries are summed by a whole warp
@@ -332,8 +344,8 @@ __device__ __forceinline__ void list_segments(const OutSegs& H, int32_t u, int32
 // entries is listed for k_out_weight_long instead.
 __global__ void k_out_weight_exact(const int32_t* __restrict__ V, const int32_t* __restrict__ E,
                                    const double* __restrict__ W, int32_t n, int32_t r0, int32_t r1,
-                                   double* __restrict__ outw, uint32_t* __restrict__ hub_key,
-                                   uint32_t* __restrict__ hub_val, int32_t* __restrict__ serial_rows,
+                                   double* __restrict__ outw, uint32_t* __restrict__ rank_key,
+                                   uint32_t* __restrict__ rank_val, int32_t* __restrict__ serial_rows,
                                    uint32_t* __restrict__ serial_count, int32_t* __restrict__ long_rows,
                                    uint32_t* __restrict__ long_count, OutSegs H) {
     constexpr int G = 4;
@@ -359,7 +371,7 @@ __global__ void k_out_weight_exact(const int32_t* __restrict__ V, const int32_t*
         int q;
         out_weight_row<G>(E, W, n, b, e, sub, s, c, q);
         if (u < r1 && sub == 0 && V[u + 1] - V[u] <= kOutWeightShort)
-            out_weight_store(u, s, c, q, outw, hub_key, hub_val, serial_rows, serial_count);
+            out_weight_store(u, s, c, q, outw, rank_key, rank_val, serial_rows, serial_count);
     }
 }
 
@@ -368,7 +380,7 @@ __global__ void k_out_weight_exact(const int32_t* __restrict__ V, const int32_t*
 __global__ void k_out_weight_long(const int32_t* __restrict__ V, const int32_t* __restrict__ E,
                                   const double* __restrict__ W, int32_t n, const int32_t* __restrict__ long_rows,
                                   const uint32_t* __restrict__ long_count, double* __restrict__ outw,
-                                  uint32_t* __restrict__ hub_key, uint32_t* __restrict__ hub_val,
+                                  uint32_t* __restrict__ rank_key, uint32_t* __restrict__ rank_val,
                                   int32_t* __restrict__ serial_rows, uint32_t* __restrict__ serial_count,
                                   OutSegs H) {
     const int lane = threadIdx.x & 31;
@@ -381,7 +393,7 @@ __global__ void k_out_weight_long(const int32_t* __restrict__ V, const int32_t* 
         int32_t c;
         int q;
         out_weight_row<32>(E, W, n, V[u], V[u + 1], lane, s, c, q);
-        if (lane == 0) out_weight_store(u, s, c, q, outw, hub_key, hub_val, serial_rows, serial_count);
+        if (lane == 0) out_weight_store(u, s, c, q, outw, rank_key, rank_val, serial_rows, serial_count);
     }
     // segments of the huge sources: the last segment of a source to arrive finishes it
     const uint32_t ns = *H.seg_count;
@@ -404,11 +416,11 @@ __global__ void k_out_weight_long(const int32_t* __restrict__ V, const int32_t* 
                 const int32_t tc = __ldcg(&A.c);
                 const int tq = __ldcg(&A.q);
                 if (W) {
-                    out_weight_store(u, ts, tc, tq, outw, hub_key, hub_val, serial_rows, serial_count);
+                    out_weight_store(u, ts, tc, tq, outw, rank_key, rank_val, serial_rows, serial_count);
                 } else {  // unit weights: the count
                     outw[u] = (double)tc;
-                    hub_key[u] = ~(uint32_t)tc;
-                    hub_val[u] = (uint32_t)u;
+                    rank_key[u] = rank_class(tc);
+                    rank_val[u] = (uint32_t)u;
                 }
             }
         }
@@ -435,8 +447,8 @@ __global__ void k_out_weight_serial(const int32_t* __restrict__ V, const int32_t
 // Unit weights: the out-weight sum is the count of valid entries, exact in any
 // order, so one warp counts a row.
 __global__ void k_out_degree(const int32_t* __restrict__ V, const int32_t* __restrict__ E, int32_t n, int32_t r0,
-                             int32_t r1, double* __restrict__ outw, uint32_t* __restrict__ hub_key,
-                             uint32_t* __restrict__ hub_val, OutSegs H) {
+                             int32_t r1, double* __restrict__ outw, uint32_t* __restrict__ rank_key,
+                             uint32_t* __restrict__ rank_val, OutSegs H) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -454,37 +466,17 @@ __global__ void k_out_degree(const int32_t* __restrict__ V, const int32_t* __res
         for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
         if (lane == 0) {
             outw[u] = (double)c;
-            hub_key[u] = ~(uint32_t)c;
-            hub_val[u] = (uint32_t)u;
+            rank_key[u] = rank_class(c);
+            rank_val[u] = (uint32_t)u;
         }
     }
 }
 
-__global__ void k_hub_slots(const uint32_t* __restrict__ ranked, int32_t nhub, int32_t* __restrict__ hub_ids,
-                            int32_t* __restrict__ hub_slot) {
-    for (int32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nhub; s += gridDim.x * blockDim.x) {
-        const int32_t v = (int32_t)ranked[s];
-        hub_ids[s] = v;
-        hub_slot[v] = s;
-    }
-}
-
-// Inbound entries from a hub store -(slot + 1).
-__global__ void k_encode_hubs(int32_t* __restrict__ in_col, int64_t nnz, const int32_t* __restrict__ hub_slot) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t s = hub_slot[in_col[i]];
-        if (s >= 0) in_col[i] = -(s + 1);
-    }
-}
-
-__global__ void k_decode_hubs(const int32_t* __restrict__ in_col, int64_t nnz, const int32_t* __restrict__ hub_ids,
-                              int32_t* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t c = in_col[i];
-        out[i] = c < 0 ? hub_ids[-c - 1] : c;
-    }
+// rank[v] = position of v in the ranking (ranked[0 .. n)), -1 for a vertex
+// without valid out-edges (they come last).
+__global__ void k_ranks(const uint32_t* __restrict__ ranked, int32_t n, int32_t nsrc, int32_t* __restrict__ rank) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        rank[ranked[i]] = i < nsrc ? (int32_t)i : -1;
 }
 
 // In-degree histogram and the sort keys: destination, or n for an entry whose
@@ -518,12 +510,14 @@ __global__ void k_weight_bits(const double* __restrict__ W, int64_t p0, int64_t 
         out[p] = __float_as_uint((float)sanitize_w(W[p]));
 }
 
-__global__ void k_dangling(const double* __restrict__ outw, int32_t n, int32_t* __restrict__ mask,
-                           unsigned long long* __restrict__ counts) {
-    __shared__ unsigned long long c0, c1;
-    if (threadIdx.x == 0) { c0 = 0; c1 = 0; }
+// Dangling mask, and the counts of vertices with out-weight <= 0, with out-weight
+// <= 1e-15 and with a rank (valid out-edges).
+__global__ void k_dangling(const double* __restrict__ outw, const uint32_t* __restrict__ rank_key, int32_t n,
+                           int32_t* __restrict__ mask, unsigned long long* __restrict__ counts) {
+    __shared__ unsigned long long c0, c1, c2;
+    if (threadIdx.x == 0) { c0 = 0; c1 = 0; c2 = 0; }
     __syncthreads();
-    unsigned long long a = 0, b = 0;
+    unsigned long long a = 0, b = 0, c = 0;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n;
          u += (int64_t)gridDim.x * blockDim.x) {
         const double w = outw[u];
@@ -531,27 +525,26 @@ __global__ void k_dangling(const double* __restrict__ outw, int32_t n, int32_t* 
         mask[u] = d;
         a += d;
         b += (w <= 1e-15) ? 1 : 0;
+        c += rank_key[u] != kNoRank ? 1 : 0;
     }
-    atomicAdd(&c0, a);
-    atomicAdd(&c1, b);
+    // warp sums first: one shared atomic per warp and count
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&c0, a);
+        atomicAdd(&c1, b);
+        atomicAdd(&c2, c);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         atomicAdd(&counts[0], c0);
         atomicAdd(&counts[1], c1);
+        atomicAdd(&counts[2], c2);
     }
-}
-
-// Merge-path coordinate of diagonal d over (row ends = in_row[1..n], entries).
-__device__ __forceinline__ int2 merge_search(const int32_t* __restrict__ in_row, int32_t n,
-                                             int64_t nnz, int64_t d) {
-    int64_t lo = d - nnz > 0 ? d - nnz : 0;
-    int64_t hi = d < n ? d : n;
-    while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if ((int64_t)in_row[mid + 1] <= d - mid - 1) lo = mid + 1;
-        else hi = mid;
-    }
-    return make_int2((int32_t)lo, (int32_t)(d - lo));
 }
 
 inline int grid_for(int64_t work, int per_block = kThreads) {
@@ -616,12 +609,13 @@ int radix_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_
     return EGPR_SUCC;
 }
 
-// Sorts (keys, vals) by the low `bits` bits of the keys, stable.  After the
+// Sorts (keys, vals) by `bits` bits of the keys from first_bit, stable.  After the
 // call the values are in the buffer *result_in_alt names; the keys are sorted
 // alongside except in the last pass, which writes values only.
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      int64_t len, int bits, cudaStream_t s, TmpAlloc& tmp, bool* result_in_alt,
-                     bool keys_needed = true, uint32_t* vals2 = nullptr, uint32_t* vals2_alt = nullptr) {
+                     bool keys_needed = true, uint32_t* vals2 = nullptr, uint32_t* vals2_alt = nullptr,
+                     int first_bit = 0) {
     *result_in_alt = false;
     if (len <= 1 || bits <= 0) return EGPR_SUCC;
     int rc = EGPR_SUCC;
@@ -640,7 +634,7 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_
     uint32_t* hist = tmp.get<uint32_t>((size_t)ntiles << (nine ? 9 : 8), &rc);
     if (!hist) return rc;
     uint32_t *kin = keys, *vin = vals, *kout = keys_alt, *vout = vals_alt, *v2in = vals2, *v2out = vals2_alt;
-    int shift = 0;
+    int shift = first_bit;
     for (int p = 0; p < passes; ++p) {
         const bool last = p == passes - 1 && !keys_needed;
         if (p < nine)
@@ -684,138 +678,228 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t len, cudaStrea
     return rc;
 }
 
-// The sweep's copy of the inbound CSR: every row keeps its entries (hub-encoded,
-// in the order of in_col) and a row without entries gets one placeholder entry
-// that reads a carried value of 0 (hub slot nhub).  One warp per row.
-__global__ void k_build_sweep_cols(const int32_t* __restrict__ in_row, const int32_t* __restrict__ in_col,
-                                   const float* __restrict__ in_w, int32_t n, const int32_t* __restrict__ sw_row,
-                                   int32_t* __restrict__ sw_col, float* __restrict__ sw_w, int32_t zero_code) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = warp; r < n; r += nwarps) {
-        const int32_t b = in_row[r], e = in_row[r + 1], o = sw_row[r];
-        if (e == b) {
-            if (lane == 0) {
-                sw_col[o] = zero_code;
-                if (sw_w) sw_w[o] = 0.f;
-            }
-            continue;
-        }
-        for (int32_t p = lane; p < e - b; p += 32) {
-            sw_col[o + p] = in_col[b + p];
-            if (sw_w) sw_w[o + p] = in_w[b + p];
-        }
+// ---- the sweep's layout -----------------------------------------------------------
+// Block and index of every inbound entry's source: (rank / kBlockSrc) in the high
+// bits, rank % kBlockSrc in the low kBlockBits (one-block layout: the rank).
+__global__ void k_source_codes(const int32_t* in_col, int64_t nnz, const int32_t* __restrict__ rank,
+                               int32_t blocked, uint32_t* code) {  // code may be in_col  // code may be in_col
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)rank[in_col[i]];
+        code[i] = blocked ? ((r / (uint32_t)kBlockSrc) << kBlockBits) | (r % (uint32_t)kBlockSrc) : r;
     }
 }
 
-// max(1, length of row r); 0 for the closing slot r = n.
-__global__ void k_row_len1(const int32_t* __restrict__ in_row, int32_t n, uint32_t* __restrict__ out) {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x)
-        out[r] = r < n ? (uint32_t)max(1, in_row[r + 1] - in_row[r]) : 0u;
-}
-
-// sw_row[n+1 .. n+7] = sw_row[n] (bulk reads of row data may run past n).
-__global__ void k_pad_tail(int32_t* sw_row, int32_t n) {
-    if (threadIdx.x > 0 && threadIdx.x < 8) sw_row[(int64_t)n + threadIdx.x] = sw_row[n];
-}
-
-// For the ideal boundary d = i * cap: the row r whose cost range holds d
-// (cost of the start of row r = sw_row[r] + R * r), the offset of d into the
-// row's entries, the row's start and its length.
-__global__ void k_chunk_cuts(const int32_t* __restrict__ sw_row, int32_t n, int64_t R, int64_t cap, int32_t ideal,
-                             int4* __restrict__ out) {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= ideal; i += gridDim.x * blockDim.x) {
-        const int64_t d = (int64_t)i * cap;
-        int32_t lo = 0, hi = n - 1;  // largest r with sw_row[r] + R*r <= d
+// First entry of every block in the code-sorted entries (nblocks + 1 values).
+__global__ void k_block_starts(const uint32_t* __restrict__ code, int32_t nnz, int32_t nblocks,
+                               int32_t* __restrict__ start) {
+    for (int32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= nblocks; b += gridDim.x * blockDim.x) {
+        int32_t lo = 0, hi = nnz;  // first entry of a block >= b
+        if (b == nblocks) lo = nnz;
         while (lo < hi) {
-            const int32_t mid = lo + ((hi - lo + 1) >> 1);
-            if ((int64_t)sw_row[mid] + R * mid <= d) lo = mid;
-            else hi = mid - 1;
+            const int32_t mid = lo + ((hi - lo) >> 1);
+            if ((int32_t)(code[mid] >> kBlockBits) < b) lo = mid + 1;
+            else hi = mid;
         }
-        const int64_t off = d - ((int64_t)sw_row[lo] + R * lo);
-        const int32_t len = sw_row[lo + 1] - sw_row[lo];
-        out[i] = make_int4(lo, (int32_t)(off < (int64_t)len ? off : (int64_t)len), sw_row[lo], len);
+        start[b] = lo;
     }
 }
 
-// Every row ends on an entry; mark it in the tile of the chunk that holds it.
-__global__ void k_tile_marks(const int32_t* __restrict__ sw_row, int32_t n, const int32_t* __restrict__ cstart,
-                             const int32_t* __restrict__ ctile, int32_t nch, uint32_t* __restrict__ bits,
-                             int32_t* __restrict__ trow) {
-    for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const int32_t p = sw_row[r + 1] - 1;
-        int32_t lo = 0, hi = nch - 1;  // last chunk starting at or before p
-        while (lo < hi) {
-            const int32_t mid = lo + ((hi - lo + 1) >> 1);
-            if (cstart[mid] <= p) lo = mid;
-            else hi = mid - 1;
-        }
-        const int32_t q = p - (cstart[lo] & ~7);
-        const int32_t t = ctile[lo] + q / kTileItems, i = q % kTileItems;
-        atomicOr(&bits[(size_t)t * kTileWords + (i >> 5)], 1u << (i & 31));
-        atomicMin(&trow[t], r);
+__device__ __forceinline__ int32_t block_of_tile(const int32_t* __restrict__ block_tile, int32_t nblocks, int32_t t) {
+    int32_t lo = 0, hi = nblocks - 1;  // the last block whose first tile is at or before t (no block is empty)
+    while (lo < hi) {
+        const int32_t mid = lo + ((hi - lo + 1) >> 1);
+        if (block_tile[mid] <= t) lo = mid;
+        else hi = mid - 1;
     }
+    return lo;
 }
 
-// Per lane of every tile: the marks of the lanes below it (one byte per lane).
-__global__ void k_tile_offsets(uint32_t* __restrict__ bits, int64_t ntiles) {
+// One warp per tile: indices and weights of its entries (zero-slot entries past
+// the block's last one), run-end marks, marks of the lanes below, mark count.
+__global__ void k_tiles(const uint32_t* __restrict__ code, const uint32_t* __restrict__ dst,
+                        const float* __restrict__ w_in, const int32_t* __restrict__ block_start,
+                        const int32_t* __restrict__ block_tile, int32_t nblocks, int32_t ntiles, int32_t blocked,
+                        int32_t chunk_shift, void* __restrict__ idx, float* __restrict__ w_out, uint32_t* __restrict__ bits,
+                        uint32_t* __restrict__ count) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t t = warp; t < ntiles; t += nwarps) {
-        uint32_t* w = bits + (size_t)t * kTileWords;
-        const uint32_t mine = __popc((w[lane >> 2] >> (8 * (lane & 3))) & 0xffu);
+        const int32_t b = block_of_tile(block_tile, nblocks, (int32_t)t);
+        const int32_t end = block_start[b + 1];
+        // 64-bit: a tile may reach past the last of nearly 2^31 entries
+        const int64_t i0 = block_start[b] + (t - block_tile[b]) * kTileItems + kLaneItems * lane;
+        uint32_t code8[kLaneItems], row8[kLaneItems + 1];
+        float w8[kLaneItems];
+#pragma unroll
+        for (int u = 0; u < kLaneItems; ++u) {
+            const bool in = i0 + u < end;
+            code8[u] = in ? code[i0 + u] : (blocked ? (uint32_t)kBlockSrc : 0xffffffffu);
+            row8[u] = in ? dst[i0 + u] : 0xffffffffu;
+            if (w_out) w8[u] = in ? w_in[i0 + u] : 0.f;
+        }
+        row8[kLaneItems] = i0 + kLaneItems < end ? dst[i0 + kLaneItems] : 0xffffffffu;
+        // a run ends with its row and with its chunk
+        const int32_t in_chunk = (1 << chunk_shift) - 1;
+        const bool chunk_end = (((int32_t)t - block_tile[b]) & in_chunk) == in_chunk;
+        uint32_t marks = 0u;
+#pragma unroll
+        for (int u = 0; u < kLaneItems; ++u)
+            if (i0 + u < end && (row8[u + 1] != row8[u] || (chunk_end && lane == 31 && u == kLaneItems - 1)))
+                marks |= 1u << u;
+        const uint32_t mine = __popc(marks);
         uint32_t incl = mine;
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += up;
         }
-        const uint32_t below = incl - mine;
-        uint32_t word = below;
-        word |= __shfl_down_sync(0xffffffffu, below, 1) << 8;
-        word |= __shfl_down_sync(0xffffffffu, below, 2) << 16;
-        word |= __shfl_down_sync(0xffffffffu, below, 3) << 24;
-        if ((lane & 3) == 0) w[8 + (lane >> 2)] = word;
-    }
-}
-
-// Entry i (destination dst[i]) of the inbound CSR to its place in the sweep's copy.
-__global__ void k_sweep_cols_by_entry(const uint32_t* __restrict__ dst, const int32_t* __restrict__ in_row,
-                                      const int32_t* __restrict__ in_col, const float* __restrict__ in_w, int64_t nnz,
-                                      const int32_t* __restrict__ sw_row, int32_t* __restrict__ sw_col,
-                                      float* __restrict__ sw_w) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = dst[i];
-        const int64_t o = i + (int64_t)(sw_row[r] - in_row[r]);
-        sw_col[o] = in_col[i];
-        if (sw_w) sw_w[o] = in_w[i];
-    }
-}
-
-// The placeholder entry of every empty row.
-__global__ void k_sweep_placeholders(const int32_t* __restrict__ in_row, int32_t n, const int32_t* __restrict__ sw_row,
-                                     int32_t* __restrict__ sw_col, float* __restrict__ sw_w, int32_t zero_code) {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        if (in_row[r + 1] == in_row[r]) {
-            sw_col[sw_row[r]] = zero_code;
-            if (sw_w) sw_w[sw_row[r]] = 0.f;
+        reinterpret_cast<uint16_t*>(bits + (size_t)t * kTileWords)[lane] = (uint16_t)(marks | ((incl - mine) << 8));
+        if (lane == 31) count[t] = incl;
+        const size_t o = (size_t)t * kTileItems + (size_t)(kLaneItems * lane);
+        if (blocked) {
+            uint4 p;
+            constexpr uint32_t m = (1u << kBlockBits) - 1u;
+            p.x = (code8[0] & m) | (code8[1] & m) << 16;
+            p.y = (code8[2] & m) | (code8[3] & m) << 16;
+            p.z = (code8[4] & m) | (code8[5] & m) << 16;
+            p.w = (code8[6] & m) | (code8[7] & m) << 16;
+            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(idx) + o) = p;
+        } else {
+            uint4* q = reinterpret_cast<uint4*>(static_cast<int32_t*>(idx) + o);
+            q[0] = make_uint4(code8[0], code8[1], code8[2], code8[3]);
+            q[1] = make_uint4(code8[4], code8[5], code8[6], code8[7]);
+        }
+        if (w_out) {
+            float4* q = reinterpret_cast<float4*>(w_out + o);
+            q[0] = make_float4(w8[0], w8[1], w8[2], w8[3]);
+            q[1] = make_float4(w8[4], w8[5], w8[6], w8[7]);
         }
     }
+}
+
+// Row tiles.  A row costs phase 2 about its pairs (at most one per block and one
+// per tile of its entries) plus its finishing (about four pairs' worth); costs are in units of four.  A
+// row tile is a run of 32-row groups: group g belongs to the tile its prefix of
+// the costs falls in, floor(prefix / cap), where a group counts at least
+// cap / max_groups, so no tile has more groups than that.
+__global__ void k_group_cost(const int32_t* __restrict__ in_row, int32_t n, int32_t nblocks, int32_t groups,
+                             uint32_t* __restrict__ cost) {
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g <= groups;
+         g += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t c = 0u;
+        for (int64_t r = g * kRowGroup; r < min((g + 1) * kRowGroup, (int64_t)n); ++r) {
+            const int32_t len = in_row[r + 1] - in_row[r];
+            c += (uint32_t)(min(len, nblocks) + len / kTileItems + 4);
+        }
+        cost[g] = (c + 3u) >> 2;  // group `groups` closes the scan with 0
+    }
+}
+
+__device__ __forceinline__ uint32_t row_tile_cap(const uint32_t* total, int32_t want) {
+    return *total / (uint32_t)want + 1u;
+}
+
+__global__ void k_group_floor(const uint32_t* __restrict__ cost, const uint32_t* __restrict__ total, int32_t want,
+                              int32_t max_groups, int32_t groups, uint32_t* __restrict__ out) {
+    const uint32_t least = (row_tile_cap(total, want) + (uint32_t)max_groups - 1u) / (uint32_t)max_groups;
+    for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g <= groups; g += gridDim.x * blockDim.x)
+        out[g] = g < groups ? max(cost[g], least) : 0u;
+}
+
+// 1 for a group that begins a row tile.
+__global__ void k_group_flags(const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ total, int32_t want,
+                              int32_t groups, uint32_t* __restrict__ flag) {
+    const uint32_t cap = row_tile_cap(total, want);
+    for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g <= groups; g += gridDim.x * blockDim.x)
+        flag[g] = g < groups && (g == 0 || prefix[g] / cap != prefix[g - 1] / cap) ? 1u : 0u;
+}
+
+// Row tile of every group, first row of every row tile.
+__global__ void k_row_tiles(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ before,
+                            int32_t groups, int32_t n, int32_t* __restrict__ group_tile,
+                            int32_t* __restrict__ row_tile) {
+    for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += gridDim.x * blockDim.x) {
+        const int32_t q = (int32_t)(before[g] + flag[g]) - 1;
+        group_tile[g] = q;
+        if (flag[g]) row_tile[q] = g * kRowGroup;
+        if (g == groups - 1) row_tile[q + 1] = n;
+    }
+}
+
+// One warp per tile: the row of each of its pairs inside the row tile, and the
+// first pair of every (row tile, block) cell.  Every cell is written once: the pair
+// before the cell's first one writes it, the block's first pair the cells up to
+// its own row tile, the last one the rest (and the closing row of cells).
+__global__ void k_pair_rows(const uint32_t* __restrict__ dst, const int32_t* __restrict__ block_start,
+                            const int32_t* __restrict__ block_tile, int32_t nblocks, int32_t ntiles,
+                            const int32_t* __restrict__ group_tile, const int32_t* __restrict__ row_tile,
+                            int32_t nrow_tiles, const uint32_t* __restrict__ bits,
+                            const int32_t* __restrict__ tile_pair, uint16_t* __restrict__ pair_row,
+                            int32_t* __restrict__ cell) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t t = warp; t < ntiles; t += nwarps) {
+        const int32_t b = block_of_tile(block_tile, nblocks, (int32_t)t);
+        const int32_t end = block_start[b + 1];
+        const int64_t i0 = block_start[b] + (t - block_tile[b]) * kTileItems + kLaneItems * lane;
+        const uint32_t mw = reinterpret_cast<const uint16_t*>(bits + (size_t)t * kTileWords)[lane];
+        int32_t k = tile_pair[t] + (int32_t)(mw >> 8);
+        for (int u = 0; u < kLaneItems; ++u) {
+            if (!(mw & (1u << u))) continue;
+            const uint32_t r = dst[i0 + u];
+            const bool last = i0 + u + 1 >= end;
+            const int32_t q0 = group_tile[r / kRowGroup];
+            pair_row[k] = (uint16_t)(r - (uint32_t)row_tile[q0]);
+            if (k == tile_pair[block_tile[b]])
+                for (int32_t q = 0; q <= q0; ++q) cell[(size_t)q * nblocks + b] = k;
+            const int32_t q1 = last ? nrow_tiles : group_tile[dst[i0 + u + 1] / kRowGroup];
+            for (int32_t q = q0 + 1; q <= q1; ++q) cell[(size_t)q * nblocks + b] = k + 1;
+            ++k;
+        }
+    }
+}
+
+// Steps of every (row tile, block) cell; 0 for the closing slot.
+__global__ void k_cell_steps(const int32_t* __restrict__ cell, int64_t cells, int32_t nblocks,
+                             uint32_t* __restrict__ count) {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c <= cells; c += (int64_t)gridDim.x * blockDim.x)
+        count[c] = c < cells ? (uint32_t)((cell[c + nblocks] - cell[c] + kStepPairs - 1) / kStepPairs) : 0u;
+}
+
+__global__ void k_steps(const int32_t* __restrict__ cell, int64_t cells, int32_t nblocks,
+                        const uint32_t* __restrict__ first, int2* __restrict__ steps, int32_t* __restrict__ row_step) {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c <= cells; c += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t at = first[c];
+        if (c % nblocks == 0) row_step[c / nblocks] = (int32_t)at;
+        if (c == cells) continue;
+        const int32_t e = cell[c + nblocks];
+        for (int32_t k = cell[c]; k < e; k += kStepPairs) steps[at++] = make_int2(k, min(kStepPairs, e - k));
+    }
+}
+
+__global__ void k_gather_i32(const int32_t* __restrict__ src, const int32_t* __restrict__ at, int32_t count,
+                             int32_t* __restrict__ out) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) out[i] = src[at[i]];
+}
+
+void expand_rows(const int32_t* row, int32_t n, int32_t* dst, cudaStream_t s) {
+    k_expand_src<<<grid_for((int64_t)n * 32), kThreads, 0, s>>>(row, n, dst);
 }
 
 // Defaults of a graph's layout parameters (egpr_graph_set_tuning and
 // egpr_graph_autotune change them per graph).
 int default_chunks_per_warp() {
     static const int v = [] {
-        const char* e = std::getenv("EGPR_CHUNKS_PER_WARP");  // queue granularity
+        const char* e = std::getenv("EGPR_CHUNKS_PER_WARP");  // row tiles per resident warp
         const int x = e ? std::atoi(e) : 8;
         return x >= 1 && x <= 64 ? x : 8;
     }();
     return v;
 }
 
-// Cost of finishing one row, in entries (a row costs its entries plus this).
+// Cost of one pair, in entries, when phase 1 is cut into CTA shares.
 int default_row_cost() {
     static const int v = [] {
         const char* e = std::getenv("EGPR_ROW_COST");
@@ -825,211 +909,160 @@ int default_row_cost() {
     return v;
 }
 
-// The sweep's work layout, built on the device (the host only sees the chunk
-// boundaries):
-//   * sw_row / sw_col / sw_w: the inbound CSR with a placeholder entry in every
-//     empty row, so that every row ends on an entry of its own;
-//   * chunks: boundaries at multiples of a cost cap along the rows, where a
-//     row costs its entries plus the graph's row cost; a boundary moves back to the
-//     start of its row unless that row began before the previous boundary (a
-//     row longer than a chunk), which is then cut (a span: its chunks add
-//     pieces to the span's accumulator and the sweep finishes the row when the
-//     launch ends); every cut leaves at least one entry on each side;
-//   * warp tiles: chunk c covers tiles of kTileItems entries from
-//     (start & ~7); per tile a 256-bit mask of the entries that end a row, per
-//     lane the number of marks in the lanes below it, and the first row a mark
-//     of the tile ends (the k-th mark of a tile ends row tile_row + k, since
-//     every row has an entry).
-// Chunks are stored costliest first, which is their queue order.
-// The layout's tables (row offsets, chunks, tile masks, span links), which
-// need in_row only; the entries follow in build_sweep_entries.
-int build_sweep_tables(egpr_graph* g, int32_t resident_warps, cudaStream_t s) {
+// (row tile, block) cells above which the blocks are given up: graphs of more than
+// about 3 * 10^8 vertices, whose cells would hold fewer pairs than a step costs.
+// EGPR_MAX_CELLS lowers it (tests).
+int64_t max_pair_cells() {
+    const char* e = std::getenv("EGPR_MAX_CELLS");
+    const long long x = e ? std::atoll(e) : 0;
+    return x > 0 ? (int64_t)x : (int64_t)1 << 28;
+}
+
+// Builds the sweep's layout (see GraphDev) from the inbound entries in
+// destination order: src (sources) in `code`, destinations in `dst`, weights in
+// `w` (NULL: unit weights).  The three arrays and their *_alt counterparts are
+// scratch of nnz entries that the sort overwrites; code may equal in_col's copy.
+int build_sweep_layout(egpr_graph* g, uint32_t* code, uint32_t* dst, uint32_t* w, uint32_t* code_alt,
+                       uint32_t* dst_alt, uint32_t* w_alt, TmpAlloc& tmp, cudaStream_t s) {
     const int32_t n = g->n;
+    const int32_t nnz = (int32_t)g->nnz;
+    int rc = EGPR_SUCC;
+    if (nnz <= 0 || g->nsrc <= 0) {
+        g->nblocks = 0;
+        g->h_block_tile.assign(1, 0);
+        g->h_block_pair.assign(1, 0);
+        g->nrow_tiles = 0;
+        return EGPR_SUCC;
+    }
+    // row tiles: a quarter of tune_cpw per resident CTA of phase 2 (fewer where they would
+    // have less than kMinTileRows rows), of up to four times the mean number of rows
+    const int32_t want = (int32_t)std::max<int64_t>(
+        1, std::min<int64_t>((int64_t)sweep_grid() * kRowTilesPerSm * std::max(1, g->tune_cpw) / 4,
+                             ((int64_t)n + kMinTileRows - 1) / kMinTileRows));
+    int32_t max_rows = kMinTileRows;
+    while (max_rows < kMaxTileRows && (int64_t)max_rows * want < 4 * (int64_t)n) max_rows = std::min(2 * max_rows, kMaxTileRows);
+    const int32_t groups = (n + kRowGroup - 1) / kRowGroup;
+    int32_t nb = (g->nsrc + kBlockSrc - 1) / kBlockSrc;
+    uint32_t* d_gcost = tmp.get<uint32_t>((size_t)groups + 1, &rc);
+    uint32_t* d_gpre = tmp.get<uint32_t>((size_t)groups + 1, &rc);
+    uint32_t* d_gfloor = tmp.get<uint32_t>((size_t)groups + 1, &rc);
+    uint32_t* d_gflag = tmp.get<uint32_t>((size_t)groups + 1, &rc);
+    int32_t* d_gtile = tmp.get<int32_t>((size_t)groups, &rc);
+    int32_t* d_rtile = tmp.get<int32_t>((size_t)groups + 1, &rc);
+    if (rc) return rc;
+    k_group_cost<<<grid_for((int64_t)groups + 1), kThreads, 0, s>>>(g->in_row.as<int32_t>(), n, nb, groups, d_gcost);
+    if ((rc = exclusive_scan_u32(d_gcost, d_gpre, (int64_t)groups + 1, s))) return rc;
+    k_group_floor<<<grid_for(groups + 1), kThreads, 0, s>>>(d_gcost, d_gpre + groups, want, max_rows / kRowGroup, groups,
+                                                            d_gfloor);
+    uint32_t* d_fpre = reinterpret_cast<uint32_t*>(d_rtile);  // free until k_row_tiles
+    if ((rc = exclusive_scan_u32(d_gfloor, d_fpre, (int64_t)groups + 1, s))) return rc;
+    k_group_flags<<<grid_for(groups + 1), kThreads, 0, s>>>(d_fpre, d_gpre + groups, want, groups, d_gflag);
+    if ((rc = exclusive_scan_u32(d_gflag, d_gfloor, (int64_t)groups + 1, s))) return rc;
+    k_row_tiles<<<grid_for(groups), kThreads, 0, s>>>(d_gflag, d_gfloor, groups, n, d_gtile, d_rtile);
+    uint32_t nrt_u = 0;
+    if ((rc = cuda_ok(cudaMemcpyAsync(&nrt_u, d_gfloor + groups, sizeof(nrt_u), cudaMemcpyDeviceToHost, s), "D2H row tiles")) ||
+        (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")))
+        return rc;
+    const int32_t nrt = (int32_t)nrt_u;
+    const bool blocked = (int64_t)nb * ((int64_t)nrt + 1) <= max_pair_cells();
+    if (!blocked) nb = 1;
+    g->nblocks = nb;
+    g->nrow_tiles = nrt;
+    g->global_block = blocked ? 0 : 1;
+    g->max_tile_rows = max_rows;
+    // chunks of four tiles where every warp still gets several of them
+    g->chunk_shift = nnz >= 2 * sweep_resident_warps() * (4 * kTileItems) ? 2 : 0;
+    k_source_codes<<<grid_for(nnz), kThreads, 0, s>>>(reinterpret_cast<const int32_t*>(code), nnz,
+                                                      g->rank.as<int32_t>(), blocked ? 1 : 0, code);
+    int bits = 0;
+    while (((nb - 1) >> bits) != 0) ++bits;
+    bool alt = false;
+    if ((rc = radix_sort_pairs(code, dst, code_alt, dst_alt, nnz, bits, s, tmp, &alt, true, w, w_alt, kBlockBits)))
+        return rc;
+    if (alt) {
+        std::swap(code, code_alt);
+        std::swap(dst, dst_alt);
+        std::swap(w, w_alt);
+    }
+    int32_t* d_start = tmp.get<int32_t>((size_t)nb + 1, &rc);
+    int32_t* d_btile = tmp.get<int32_t>((size_t)nb + 1, &rc);
+    int32_t* d_bpair = tmp.get<int32_t>((size_t)nb + 1, &rc);
+    if (rc) return rc;
+    std::vector<int32_t> start((size_t)nb + 1);
+    if (blocked) {
+        k_block_starts<<<grid_for(nb + 1), kThreads, 0, s>>>(code, nnz, nb, d_start);
+        if ((rc = cuda_ok(cudaMemcpyAsync(start.data(), d_start, start.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H block starts")) ||
+            (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")))
+            return rc;
+    } else {
+        start[0] = 0;
+        start[1] = nnz;
+        if ((rc = cuda_ok(cudaMemcpyAsync(d_start, start.data(), start.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s), "H2D block starts")))
+            return rc;
+    }
+    std::vector<int32_t>& btile = g->h_block_tile;
+    btile.assign((size_t)nb + 1, 0);
+    for (int32_t b = 0; b < nb; ++b)
+        btile[(size_t)b + 1] = btile[(size_t)b] +
+                               (int32_t)(((int64_t)start[(size_t)b + 1] - start[(size_t)b] + kTileItems - 1) / kTileItems);
+    const int32_t ntiles = btile[(size_t)nb];
+    const size_t entries = (size_t)ntiles * kTileItems;
+    const int64_t cells = (int64_t)nrt * nb;
+    uint32_t* d_count = tmp.get<uint32_t>((size_t)ntiles + 1, &rc);
+    int32_t* d_cell = tmp.get<int32_t>((size_t)cells + (size_t)nb, &rc);  // [row tile][block], closed by a row
+    uint32_t* d_first = tmp.get<uint32_t>((size_t)cells + 1, &rc);
+    if (rc || (rc = g->idx.alloc(entries * (blocked ? sizeof(uint16_t) : sizeof(int32_t)))) ||
+        (g->weighted && (rc = g->sw_w.alloc(entries * sizeof(float)))) ||
+        (rc = g->tile_bits.alloc((size_t)ntiles * kTileWords * sizeof(uint32_t))) ||
+        (rc = g->tile_pair.alloc(((size_t)ntiles + 1) * sizeof(int32_t))) ||
+        (rc = g->row_tile.alloc(((size_t)nrt + 1) * sizeof(int32_t))) ||
+        (rc = g->row_step.alloc(((size_t)nrt + 1) * sizeof(int32_t))))
+        return rc;
+    if ((rc = cuda_ok(cudaMemcpyAsync(g->row_tile.p, d_rtile, ((size_t)nrt + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s), "row tiles")) ||
+        (rc = cuda_ok(cudaMemcpyAsync(d_btile, btile.data(), btile.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s), "H2D block tiles")) ||
+        (rc = cuda_ok(cudaMemsetAsync(d_count + ntiles, 0, sizeof(uint32_t), s), "memset")))
+        return rc;
+    k_tiles<<<grid_for((int64_t)ntiles * 32), kThreads, 0, s>>>(
+        code, dst, reinterpret_cast<const float*>(w), d_start, d_btile, nb, ntiles, blocked ? 1 : 0, g->chunk_shift, g->idx.p,
+        g->weighted ? g->sw_w.as<float>() : nullptr, g->tile_bits.as<uint32_t>(), d_count);
+    if ((rc = exclusive_scan_u32(d_count, g->tile_pair.as<uint32_t>(), (int64_t)ntiles + 1, s))) return rc;
+    k_gather_i32<<<grid_for(nb + 1), kThreads, 0, s>>>(g->tile_pair.as<int32_t>(), d_btile, nb + 1, d_bpair);
+    g->h_block_pair.assign((size_t)nb + 1, 0);
+    if ((rc = cuda_ok(cudaMemcpyAsync(g->h_block_pair.data(), d_bpair, ((size_t)nb + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H pairs")) ||
+        (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")))
+        return rc;
+    const size_t npairs = (size_t)g->h_block_pair[(size_t)nb];
+    if ((rc = g->pair_row.alloc(npairs * sizeof(uint16_t))) || (rc = g->pairs.alloc(npairs * sizeof(double)))) return rc;
+    k_pair_rows<<<grid_for((int64_t)ntiles * 32), kThreads, 0, s>>>(
+        dst, d_start, d_btile, nb, ntiles, d_gtile, d_rtile, nrt, g->tile_bits.as<uint32_t>(),
+        g->tile_pair.as<int32_t>(), g->pair_row.as<uint16_t>(), d_cell);
+    k_cell_steps<<<grid_for(cells + 1), kThreads, 0, s>>>(d_cell, cells, nb, d_first);
+    if ((rc = exclusive_scan_u32(d_first, d_first, cells + 1, s))) return rc;
+    uint32_t nsteps = 0;
+    if ((rc = cuda_ok(cudaMemcpyAsync(&nsteps, d_first + cells, sizeof(nsteps), cudaMemcpyDeviceToHost, s), "D2H steps")) ||
+        (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")) || (rc = g->steps.alloc((size_t)nsteps * sizeof(int2))))
+        return rc;
+    k_steps<<<grid_for(cells + 1), kThreads, 0, s>>>(d_cell, cells, nb, d_first, g->steps.as<int2>(), g->row_step.as<int32_t>());
+    if ((rc = cuda_ok(cudaGetLastError(), "sweep layout"))) return rc;
+    return cuda_ok(cudaStreamSynchronize(s), "sweep layout");
+}
+
+int rebuild_sweep_layout(egpr_graph* g, cudaStream_t s) {
     TmpAlloc tmp(s);
     int rc = EGPR_SUCC;
-    // placeholder offsets: sw_row = exclusive scan of max(1, row length)
-    uint32_t* len1 = tmp.get<uint32_t>((size_t)n + 1, &rc);
-    if (rc || (rc = g->sw_row.alloc(((size_t)n + 8) * sizeof(int32_t)))) return rc;
-    k_row_len1<<<grid_for((int64_t)n + 1), kThreads, 0, s>>>(g->in_row.as<int32_t>(), n, len1);
-    if ((rc = exclusive_scan_u32(len1, reinterpret_cast<uint32_t*>(g->sw_row.as<int32_t>()), (int64_t)n + 1, s))) return rc;
-    k_pad_tail<<<1, 32, 0, s>>>(g->sw_row.as<int32_t>(), n);
-    uint32_t nnz_u = 0;
-    if ((rc = cuda_ok(cudaMemcpyAsync(&nnz_u, g->sw_row.as<int32_t>() + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "D2H sweep entries")) ||
-        (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")))
-        return rc;
-    if ((int64_t)nnz_u > (int64_t)INT32_MAX - 4096) return EGPR_UNSUPPORTED_GRAPH;
-    const int32_t nnz = (int32_t)nnz_u;
-    g->sw_nnz = nnz;
-    // chunk boundaries at ideal costs d_i = i * cap
-    const int64_t R = g->tune_rc;
-    const int64_t warps = std::max(1, resident_warps);
-    const int64_t total = (int64_t)nnz + R * (int64_t)n;
-    const int64_t cpw = std::max(1, g->tune_cpw);
-    int64_t cap = (total + warps * cpw - 1) / (warps * cpw);
-    cap = std::min<int64_t>(std::max<int64_t>(kTileItems + R + 1, cap), 1 << 24);
-    const int64_t ideal = std::max<int64_t>(1, (total + cap - 1) / cap);
-    int4* d_cut = tmp.get<int4>((size_t)ideal + 1, &rc);
+    const size_t nnz = (size_t)std::max<int64_t>(g->nnz, 1);
+    uint32_t* code = tmp.get<uint32_t>(nnz, &rc);
+    uint32_t* code2 = tmp.get<uint32_t>(nnz, &rc);
+    uint32_t* dst = tmp.get<uint32_t>(nnz, &rc);
+    uint32_t* dst2 = tmp.get<uint32_t>(nnz, &rc);
+    uint32_t* w = g->weighted ? tmp.get<uint32_t>(nnz, &rc) : nullptr;
+    uint32_t* w2 = g->weighted ? tmp.get<uint32_t>(nnz, &rc) : nullptr;
     if (rc) return rc;
-    k_chunk_cuts<<<grid_for(ideal + 1), kThreads, 0, s>>>(g->sw_row.as<int32_t>(), n, R, cap, (int32_t)ideal, d_cut);
-    std::vector<int4> cut((size_t)ideal + 1);
-    if ((rc = cuda_ok(cudaMemcpyAsync(cut.data(), d_cut, cut.size() * sizeof(int4), cudaMemcpyDeviceToHost, s), "D2H chunk cuts")) ||
-        (rc = cuda_ok(cudaStreamSynchronize(s), "sweep layout")))
+    expand_rows(g->in_row.as<int32_t>(), g->n, reinterpret_cast<int32_t*>(dst), s);
+    if ((rc = cuda_ok(cudaMemcpyAsync(code, g->in_col.p, (size_t)g->nnz * sizeof(int32_t), cudaMemcpyDeviceToDevice, s), "sources")) ||
+        (w && (rc = cuda_ok(cudaMemcpyAsync(w, g->in_w.p, (size_t)g->nnz * sizeof(float), cudaMemcpyDeviceToDevice, s), "weights"))))
         return rc;
-    struct B {
-        int32_t r, k, rs;  // boundary: row, entry, start of that row
-    };
-    std::vector<B> bs;
-    bs.push_back(B{0, 0, 0});
-    for (int64_t i = 1; i < ideal; ++i) {
-        const int4 c = cut[(size_t)i];  // (row, offset into the row, row start, row length)
-        const B& p = bs.back();
-        if (c.z > p.k) {
-            bs.push_back(B{c.x, c.z, c.z});  // the row's start
-        } else if (c.w >= 2) {
-            const int32_t k = c.z + std::min(std::max(c.y, 1), c.w - 1);  // a cut inside a long row
-            if (c.x == p.r && k > p.k) bs.push_back(B{c.x, k, c.z});
-        }
-    }
-    bs.push_back(B{n, nnz, nnz});
-    const int32_t nch = (int32_t)bs.size() - 1;
-    std::vector<Chunk>& ch = g->plan.h_chunks;
-    ch.assign((size_t)nch, Chunk{});
-    std::vector<int32_t> cstart((size_t)nch), ctile((size_t)nch);
-    int64_t ntiles = 0;
-    for (int32_t c = 0; c < nch; ++c) {
-        const B& a = bs[(size_t)c];
-        const B& b = bs[(size_t)c + 1];
-        const int32_t t0 = a.k & ~7;
-        const int32_t nt = std::max<int32_t>(1, (b.k - t0 + kTileItems - 1) / kTileItems);
-        Chunk& k = ch[(size_t)c];
-        const bool head = a.r < n && a.k > a.rs;
-        const bool tail = b.r < n && b.k > b.rs;
-        int32_t f = 0;
-        if (head) f |= kHasHead;
-        if (tail) f |= kHasTail;
-        if (head && tail && a.r == b.r) f |= kInterior;
-        k.flags = f;
-        k.tile_begin = (int32_t)ntiles;
-        k.tile_end = (int32_t)(ntiles + nt);
-        k.nnz_begin = a.k;
-        k.nnz_end = b.k;
-        k.row_end = b.r;
-        k.pad = (int32_t)std::min<int64_t>((int64_t)(b.k - a.k) + R * (int64_t)(b.r - a.r + 1), INT32_MAX);  // cost
-        k.graph = 0;
-        k.tail_row = tail ? b.r : -1;
-        k.head_ta = -1;
-        k.tail_tb = -1;
-        k.pad2 = 0;
-        cstart[(size_t)c] = a.k;
-        ctile[(size_t)c] = (int32_t)ntiles;
-        ntiles += nt;
-    }
-    if (ntiles > INT32_MAX / 2) return EGPR_UNSUPPORTED_GRAPH;
-    g->ntiles = (int32_t)ntiles;
-    // tile tables: marks by row ends, then per-lane offsets
-    int32_t* d_cstart = tmp.get<int32_t>((size_t)nch, &rc);
-    int32_t* d_ctile = tmp.get<int32_t>((size_t)nch, &rc);
-    if (rc || (rc = g->tile_bits.alloc((size_t)ntiles * kTileWords * sizeof(uint32_t))) ||
-        (rc = g->tile_row.alloc((size_t)ntiles * sizeof(int32_t))))
-        return rc;
-    if ((rc = cuda_ok(cudaMemcpyAsync(d_cstart, cstart.data(), (size_t)nch * sizeof(int32_t), cudaMemcpyHostToDevice, s), "H2D chunk starts")) ||
-        (rc = cuda_ok(cudaMemcpyAsync(d_ctile, ctile.data(), (size_t)nch * sizeof(int32_t), cudaMemcpyHostToDevice, s), "H2D chunk tiles")) ||
-        (rc = cuda_ok(cudaMemsetAsync(g->tile_bits.p, 0, g->tile_bits.bytes, s), "memset")) ||
-        (rc = cuda_ok(cudaMemsetAsync(g->tile_row.p, 0x7f, g->tile_row.bytes, s), "memset")))
-        return rc;
-    k_tile_marks<<<grid_for(n), kThreads, 0, s>>>(g->sw_row.as<int32_t>(), n, d_cstart, d_ctile, nch,
-                                                   g->tile_bits.as<uint32_t>(), g->tile_row.as<int32_t>());
-    k_tile_offsets<<<grid_for(ntiles * 32), kThreads, 0, s>>>(g->tile_bits.as<uint32_t>(), ntiles);
-    // span links (row order), then the queue order: costliest chunks first
-    g->plan.h_spans.clear();
-    for (int32_t c = 0; c < nch; ++c) {
-        Chunk& k = ch[(size_t)c];
-        if (k.flags & kHasHead) k.head_ta = (ch[(size_t)c - 1].flags & kInterior) ? ch[(size_t)c - 1].head_ta : c - 1;
-        if ((k.flags & kHasTail) && !(k.flags & kInterior)) g->plan.h_spans.push_back(c);
-    }
-    for (int32_t c = nch - 1; c >= 0; --c) {
-        Chunk& k = ch[(size_t)c];
-        if (k.flags & kHasTail) k.tail_tb = (ch[(size_t)c + 1].flags & kInterior) ? ch[(size_t)c + 1].tail_tb : c + 1;
-    }
-    {
-        // chunks of the span each chunk adds to (its head row's, its tail row's),
-        // counted before the renumbering
-        std::vector<int32_t> hparts((size_t)nch, 0), tparts((size_t)nch, 0);
-        for (int32_t c = 0; c < nch; ++c) {
-            const Chunk& k = ch[(size_t)c];
-            if (k.flags & kInterior) hparts[(size_t)c] = k.tail_tb - k.head_ta + 1;
-            else if (k.flags & kHasHead) hparts[(size_t)c] = c - k.head_ta + 1;
-            if ((k.flags & kHasTail) && !(k.flags & kInterior)) tparts[(size_t)c] = k.tail_tb - c + 1;
-        }
-        // costliest first: a stable counting sort over 4096 cost classes (the
-        // order only needs to be roughly by cost, and a comparison sort of the
-        // ~28K records costs milliseconds of host time)
-        std::vector<int32_t> perm((size_t)nch), pos_of((size_t)nch);
-        {
-            int64_t cmax = 1;
-            for (int32_t c = 0; c < nch; ++c) cmax = std::max<int64_t>(cmax, ch[(size_t)c].pad);
-            constexpr int kClasses = 4096;
-            std::vector<int32_t> start(kClasses + 1, 0);
-            auto cls = [&](int32_t c) {
-                return kClasses - 1 - (int32_t)(((int64_t)ch[(size_t)c].pad * (kClasses - 1)) / cmax);
-            };
-            for (int32_t c = 0; c < nch; ++c) start[(size_t)cls(c) + 1] += 1;
-            for (int i = 0; i < kClasses; ++i) start[(size_t)i + 1] += start[(size_t)i];
-            for (int32_t c = 0; c < nch; ++c) perm[(size_t)start[(size_t)cls(c)]++] = c;
-        }
-        for (int32_t i = 0; i < nch; ++i) pos_of[(size_t)perm[(size_t)i]] = i;
-        std::vector<Chunk> sorted((size_t)nch);
-        for (int32_t i = 0; i < nch; ++i) {
-            Chunk k = ch[(size_t)perm[(size_t)i]];
-            if (k.head_ta >= 0) k.head_ta = pos_of[(size_t)k.head_ta];
-            if (k.tail_tb >= 0) k.tail_tb = pos_of[(size_t)k.tail_tb];
-            k.pad = hparts[(size_t)perm[(size_t)i]];
-            k.pad2 = tparts[(size_t)perm[(size_t)i]];
-            sorted[(size_t)i] = k;
-        }
-        ch.swap(sorted);
-        for (int32_t& sp : g->plan.h_spans) sp = pos_of[(size_t)sp];
-    }
-    // entries (a tile reads up to kTileItems + 8 entries past a chunk's start)
-    const size_t pad = (size_t)(kTileItems + 16) * sizeof(int32_t);
-    if ((rc = g->sw_col.alloc((size_t)nnz * sizeof(int32_t) + pad)) ||
-        (g->weighted && (rc = g->sw_w.alloc((size_t)nnz * sizeof(float) + pad))))
-        return rc;
-    return cuda_ok(cudaGetLastError(), "sweep tables");
-}
-
-// The layout's entries: in_col (hub codes already in place) copied behind the
-// row offsets, with a placeholder in every empty row.  Stream-ordered; the
-// tables must be complete on the device.
-int build_sweep_entries(egpr_graph* g, const uint32_t* sorted_dst, cudaStream_t s) {
-    const int32_t n = g->n;
-    const int32_t nnz = (int32_t)g->sw_nnz;
-    const size_t pad = (size_t)(kTileItems + 16) * sizeof(int32_t);
-    int rc;
-    // every entry is written below; only the padding past the last one is cleared
-    if ((rc = cuda_ok(cudaMemsetAsync(g->sw_col.as<int32_t>() + nnz, 0, pad, s), "memset"))) return rc;
-    if (g->weighted && (rc = cuda_ok(cudaMemsetAsync(g->sw_w.as<float>() + nnz, 0, pad, s), "memset"))) return rc;
-    if (sorted_dst && g->nnz > 0) {
-        // entry-parallel: entry i of row r moves by the number of empty rows before r
-        k_sweep_cols_by_entry<<<grid_for(g->nnz), kThreads, 0, s>>>(
-            sorted_dst, g->in_row.as<int32_t>(), g->in_col.as<int32_t>(), g->weighted ? g->in_w.as<float>() : nullptr,
-            g->nnz, g->sw_row.as<int32_t>(), g->sw_col.as<int32_t>(), g->weighted ? g->sw_w.as<float>() : nullptr);
-        k_sweep_placeholders<<<grid_for(n), kThreads, 0, s>>>(g->in_row.as<int32_t>(), n, g->sw_row.as<int32_t>(),
-                                                             g->sw_col.as<int32_t>(),
-                                                             g->weighted ? g->sw_w.as<float>() : nullptr, -(g->nhub + 1));
-    } else {
-        k_build_sweep_cols<<<grid_for((int64_t)n * 32), kThreads, 0, s>>>(
-            g->in_row.as<int32_t>(), g->in_col.as<int32_t>(), g->weighted ? g->in_w.as<float>() : nullptr, n,
-            g->sw_row.as<int32_t>(), g->sw_col.as<int32_t>(), g->weighted ? g->sw_w.as<float>() : nullptr,
-            -(g->nhub + 1));
-    }
-    return cuda_ok(cudaGetLastError(), "sweep entries");
-}
-
-int build_sweep_layout(egpr_graph* g, int32_t resident_warps, const uint32_t* sorted_dst, cudaStream_t s) {
-    int rc;
-    if ((rc = build_sweep_tables(g, resident_warps, s)) || (rc = build_sweep_entries(g, sorted_dst, s))) return rc;
-    return cuda_ok(cudaStreamSynchronize(s), "sweep layout");
+    return build_sweep_layout(g, code, dst, w, code2, dst2, w2, tmp, s);
 }
 
 // ---- the binned sweep's layout -------------------------------------------------
@@ -1372,7 +1405,7 @@ int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const doubl
         // weighted: the FP32 weight of every entry moves through the sort with its source
         uint32_t* wbits = W ? tmp.get<uint32_t>((size_t)m, &rc) : nullptr;
         uint32_t* wbits2 = W ? tmp.get<uint32_t>((size_t)m, &rc) : nullptr;
-        unsigned long long* counts = tmp.get<unsigned long long>(2, &rc);
+        unsigned long long* counts = tmp.get<unsigned long long>(3, &rc);
         uint32_t* hkey = tmp.get<uint32_t>((size_t)n, &rc);
         uint32_t* hval = tmp.get<uint32_t>((size_t)n, &rc);
         uint32_t* hkey2 = tmp.get<uint32_t>((size_t)n, &rc);
@@ -1391,14 +1424,13 @@ int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const doubl
         segs.acc_count = tmp.get<uint32_t>(1, &rc);
         if (rc) return rc;
         if (W) cudaMemsetAsync(serial_count, 0, sizeof(uint32_t), s);
-        // in_row, hub_slot: bulk copies of a stage's rows may read up to 3 elements past the end.
         if ((rc = g->in_row.alloc(((size_t)n + 8) * sizeof(int32_t))) ||
             (rc = g->outw.alloc((size_t)n * sizeof(double))) ||
             (rc = g->dangling01.alloc((size_t)n * sizeof(int32_t))))
             return rc;
         if ((rc = upload_h2d(dV, V, ((size_t)n + 1) * sizeof(int32_t), v_locked, s, "H2D offsets"))) return rc;
         cudaMemsetAsync(indeg, 0, ((size_t)n + 1) * sizeof(uint32_t), s);
-        cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), s);
+        cudaMemsetAsync(counts, 0, 3 * sizeof(unsigned long long), s);
         // the sort carries each entry's source (written from the offsets alone,
         // while E is still arriving) and, when weighted, its FP32 weight
         // (converted as each piece of W arrives), so no gather follows it
@@ -1473,14 +1505,18 @@ int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const doubl
         }
         if ((rc = exclusive_scan_u32(indeg, reinterpret_cast<uint32_t*>(g->in_row.as<int32_t>()), (int64_t)n + 1, s)))
             return rc;
-        const uint32_t* sorted_dst = nullptr;  // destination of every inbound entry, in entry order
+        k_dangling<<<grid_for(n), kThreads, 0, s>>>(g->outw.as<double>(), hkey, n, g->dangling01.as<int32_t>(), counts);
         int32_t nnz32 = 0;
+        unsigned long long hc[3] = {0, 0, 0};
         if ((rc = cuda_ok(cudaMemcpyAsync(&nnz32, g->in_row.as<int32_t>() + n, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H nnz")) ||
+            (rc = cuda_ok(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s), "D2H counts")) ||
             (rc = cuda_ok(cudaStreamSynchronize(s), "preparation")))
             return rc;
         g->nnz = nnz32;
+        g->n_dangling = (int32_t)hc[0];
+        g->n_dangling_solve = (int32_t)hc[1];
+        g->nsrc = (int32_t)hc[2];
         const int64_t nnz = g->nnz;
-        // Padding: a stage's bulk copy reads up to 3 entries past the end.
         const size_t pad = 16 * sizeof(int32_t);
         if ((rc = g->in_col.alloc((size_t)std::max<int64_t>(nnz, 1) * sizeof(int32_t) + pad)))
             return rc;
@@ -1495,79 +1531,30 @@ int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const doubl
             bool alt = false;
             if ((rc = radix_sort_pairs(keys, vals, keys2, vals2, m, bits, s, tmp, &alt, true, wbits, wbits2)))
                 return rc;
-            const uint32_t* sorted_vals = alt ? vals2 : vals;
-            sorted_dst = alt ? keys2 : keys;
-            if (nnz > 0 && (rc = cuda_ok(cudaMemcpyAsync(g->in_col.p, sorted_vals, (size_t)nnz * sizeof(int32_t),
+            if (alt) {
+                std::swap(keys, keys2);
+                std::swap(vals, vals2);
+                std::swap(wbits, wbits2);
+            }
+            if (nnz > 0 && (rc = cuda_ok(cudaMemcpyAsync(g->in_col.p, vals, (size_t)nnz * sizeof(int32_t),
                                                          cudaMemcpyDeviceToDevice, s), "inbound sources")))
                 return rc;
             if (W && nnz > 0 &&
-                (rc = cuda_ok(cudaMemcpyAsync(g->in_w.p, alt ? wbits2 : wbits, (size_t)nnz * sizeof(float),
+                (rc = cuda_ok(cudaMemcpyAsync(g->in_w.p, wbits, (size_t)nnz * sizeof(float),
                                               cudaMemcpyDeviceToDevice, s), "inbound weights")))
                 return rc;
         }
-        // Hubs: the min(n, kHubCap) sources of largest out-degree (a multiple of 4,
-        // the granule of the shared-memory staging copy).
-        // EGPR_HUBS=N: hub cache size (0: none); at most kHubCap - 32, which leaves
-        // room for the zero slot nhub in a kHubCap-value copy.  By default 24,544
-        // hubs, and 16,352 from 2^24 vertices: the shared memory the hubs take is
-        // L1 the sweep's other loads lose, and measured on B200 the smaller cache
-        // wins once the rank vector no longer fits L2 (R-MAT scale 25 weighted:
-        // 2.02 ms per sweep with 16K hubs, 2.06 with 8K, 2.08 with 24K, 2.32 with
-        // 32K; scale 22: 0.236, 0.224, 0.222 ms with 8K, 24K, 32K)
-        const char* hub_env = std::getenv("EGPR_HUBS");
-        const int32_t hub_default = n >= (1 << 24) ? 16384 - 32 : 24576 - 32;
-        const int32_t hub_want = hub_env ? std::max(0, std::atoi(hub_env)) : hub_default;
-        g->nhub = std::min<int32_t>(std::min<int32_t>(n, hub_want), kHubCap - 32) & ~3;
-        if ((rc = g->hub_slot.alloc(((size_t)n + 8) * sizeof(int32_t))) ||
-            (rc = g->hub_ids.alloc((size_t)std::max(g->nhub + 1, 4) * sizeof(int32_t))) ||
-            (rc = cuda_ok(cudaMemsetAsync(g->hub_slot.p, 0xff, ((size_t)n + 8) * sizeof(int32_t), s), "memset")))
+        // the out-degree ranking (classes, then vertex ids)
+        bool ralt = false;
+        if ((rc = g->rank.alloc((size_t)n * sizeof(int32_t))) ||
+            (rc = radix_sort_pairs(hkey, hval, hkey2, hval2, n, 8, s, tmp, &ralt, false)))
             return rc;
-        // the out-degree ranking (descending, ties by id): the hubs of both sweeps
-        const bool want_bins = bins_wanted(n, nnz);
-        const uint32_t* ranked = nullptr;
-        if (g->nhub > 0 || want_bins) {
-            bool alt = false;
-            if ((rc = radix_sort_pairs(hkey, hval, hkey2, hval2, n, 32, s, tmp, &alt, false))) return rc;
-            ranked = alt ? hval2 : hval;
-        }
-        // the binned layout reads in_col before the hub codes go in
-        if (want_bins && (rc = build_bin_layout(g, sorted_dst, ranked, tmp, s))) return rc;
-        if (g->nhub > 0) {
-            k_hub_slots<<<grid_for(g->nhub), kThreads, 0, s>>>(ranked, g->nhub, g->hub_ids.as<int32_t>(),
-                                                               g->hub_slot.as<int32_t>());
-            if (nnz > 0)
-                k_encode_hubs<<<grid_for(nnz), kThreads, 0, s>>>(g->in_col.as<int32_t>(), nnz, g->hub_slot.as<int32_t>());
-        }
-        // hub slot nhub is the zero slot of placeholder entries; in the FP64
-        // correction sweep it reads z64[n] = 0
-        if ((rc = cuda_ok(cudaMemcpyAsync(g->hub_ids.as<int32_t>() + g->nhub, &g->n, sizeof(int32_t),
-                                          cudaMemcpyHostToDevice, s), "H2D zero slot")))
-            return rc;
-        k_dangling<<<grid_for(n), kThreads, 0, s>>>(g->outw.as<double>(), n, g->dangling01.as<int32_t>(), counts);
-        // The layout's tables need in_row only (complete since the nnz read
-        // above): they are built on a second stream while the inbound sort, the
-        // gather and the hub ranking run on s; the entries then follow on s.
-        cudaStream_t s2 = nullptr;
-        cudaEvent_t e2 = nullptr;
-        if ((rc = cuda_ok(cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking), "stream")) ||
-            (rc = cuda_ok(cudaEventCreateWithFlags(&e2, cudaEventDisableTiming), "event"))) {
-            if (s2) cudaStreamDestroy(s2);
-            return rc;
-        }
-        rc = build_sweep_tables(g, sweep_resident_warps(), s2);
-        if (!rc) rc = cuda_ok(cudaEventRecord(e2, s2), "event");
-        if (!rc) rc = cuda_ok(cudaStreamWaitEvent(s, e2, 0), "event");
-        if (!rc) rc = build_sweep_entries(g, sorted_dst, s);
-        if (rc) cudaStreamSynchronize(s2);  // nothing of s2 may outlive an early return
-        cudaEventDestroy(e2);
-        cudaStreamDestroy(s2);  // released once its work is done
-        if (rc) return rc;
-        unsigned long long hc[2] = {0, 0};
-        // a copy into pageable memory returns once it is done, after all of s above
-        if ((rc = cuda_ok(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s), "D2H counts")))
-            return rc;
-        g->n_dangling = (int32_t)hc[0];
-        g->n_dangling_solve = (int32_t)hc[1];
+        const uint32_t* ranked = ralt ? hval2 : hval;
+        k_ranks<<<grid_for(n), kThreads, 0, s>>>(ranked, n, g->nsrc, g->rank.as<int32_t>());
+        // both layouts read the destination-sorted entries, the sweep's last
+        // (its sort overwrites them)
+        if (bins_wanted(n, nnz) && (rc = build_bin_layout(g, keys, ranked, tmp, s))) return rc;
+        if ((rc = build_sweep_layout(g, vals, keys, wbits, vals2, keys2, wbits2, tmp, s))) return rc;
     }
     cudaEventRecord(g->ev1, s);
     if ((rc = cuda_ok(cudaStreamSynchronize(s), "preparation"))) return rc;
@@ -1578,17 +1565,10 @@ int prepare_graph(egpr_graph* g, const int32_t* V, const int32_t* E, const doubl
     return EGPR_SUCC;
 }
 
-// Copies in_col to the host with hub entries decoded back to source ids.
 int export_in_col(const egpr_graph* g, int32_t* host, cudaStream_t s) {
     if (g->nnz <= 0) return EGPR_SUCC;
-    int32_t* tmp = nullptr;
-    int rc = cuda_ok(cudaMallocAsync(&tmp, (size_t)g->nnz * sizeof(int32_t), s), "cudaMallocAsync (export)");
-    if (rc) return rc;
-    k_decode_hubs<<<grid_for(g->nnz), kThreads, 0, s>>>(g->in_col.as<int32_t>(), g->nnz, g->hub_ids.as<int32_t>(),
-                                                        tmp);
-    rc = cuda_ok(cudaMemcpyAsync(host, tmp, (size_t)g->nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H in_col");
-    cudaFreeAsync(tmp, s);
-    return rc;
+    return cuda_ok(cudaMemcpyAsync(host, g->in_col.p, (size_t)g->nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, s),
+                   "D2H in_col");
 }
 
 }  // namespace egpr

@@ -681,37 +681,45 @@ k_spmm(const SpmmParams* __restrict__ Pd, cudaGraphConditionalHandle cond, int32
 }
 
 // ---- layout ------------------------------------------------------------------------
-// Entry stream from the sweep's padded CSR: resolved sources and coefficients;
-// entries past the last one are placeholders.
-__global__ void k_sp_entries(const int32_t* __restrict__ sw_col, const float* __restrict__ sw_w, int64_t sw_nnz,
-                             int64_t epad, const int32_t* __restrict__ hub_ids, int32_t nhub,
-                             const double* __restrict__ outw, int32_t n, int32_t* __restrict__ src,
-                             float* __restrict__ c32, double* __restrict__ c64) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < epad; e += (int64_t)gridDim.x * blockDim.x) {
-        int32_t s = n;
-        double cf = 0.0;
-        if (e < sw_nnz) {
-            const int32_t code = sw_col[e];
-            if (code != -(nhub + 1)) {  // not a placeholder
-                s = code >= 0 ? code : hub_ids[-code - 1];
-                const double o = outw[s];
-                const double w = sw_w ? (double)sw_w[e] : 1.0;
-                cf = o <= 1e-15 ? 0.0 : w / o;
-            } else {
-                s = n;
-            }
-        }
-        src[e] = s;
+// Row lengths of the padded CSR: max(1, length of row r); 0 for the closing slot r = n.
+__global__ void k_sp_row_len(const int32_t* __restrict__ in_row, int32_t n, uint32_t* __restrict__ out) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x)
+        out[r] = r < n ? (uint32_t)max(1, in_row[r + 1] - in_row[r]) : 0u;
+}
+
+// Entry stream from the inbound CSR: entry i of row dst[i] moves by the number of
+// empty rows before it; bit 31 on the last entry of every row.
+__global__ void k_sp_entries(const int32_t* __restrict__ dst, const int32_t* __restrict__ in_row,
+                             const int32_t* __restrict__ in_col, const float* __restrict__ in_w, int64_t nnz,
+                             const int32_t* __restrict__ sw_row, const double* __restrict__ outw,
+                             int32_t* __restrict__ src, float* __restrict__ c32, double* __restrict__ c64) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t r = dst[i], s = in_col[i];
+        const int64_t e = i + (int64_t)(sw_row[r] - in_row[r]);
+        const double o = outw[s], w = in_w ? (double)in_w[i] : 1.0;
+        const double cf = o <= 1e-15 ? 0.0 : w / o;
+        src[e] = i + 1 == in_row[r + 1] ? (s | kRowEnd) : s;
         c32[e] = (float)cf;
         c64[e] = cf;
     }
 }
 
-// Bit 31 on the last entry of every row.
-__global__ void k_sp_marks(const int32_t* __restrict__ sw_row, int32_t n, int32_t* __restrict__ src) {
-    for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const int32_t e = sw_row[r + 1] - 1;
-        src[e] |= kRowEnd;
+// Placeholders: the entry of every empty row, and the entries past the last row.
+__global__ void k_sp_placeholders(const int32_t* __restrict__ in_row, const int32_t* __restrict__ sw_row, int32_t n,
+                                  int64_t sw_nnz, int64_t epad, int32_t* __restrict__ src, float* __restrict__ c32,
+                                  double* __restrict__ c64) {
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = t0; r < n; r += step) {
+        if (in_row[r + 1] != in_row[r]) continue;
+        const int32_t e = sw_row[r];
+        src[e] = n | kRowEnd;
+        c32[e] = 0.f;
+        c64[e] = 0.0;
+    }
+    for (int64_t e = sw_nnz + t0; e < epad; e += step) {
+        src[e] = n;
+        c32[e] = 0.f;
+        c64[e] = 0.0;
     }
 }
 
@@ -981,19 +989,41 @@ int grid_1d(int64_t work) {
 int build_spmm_layout(egpr_graph* g, SpmmWork& w, cudaStream_t s) {
     const int32_t n = g->n;
     const int32_t C = std::max(64, g->tune_spmm_chunk & ~31);
-    if (g->sw_nnz <= 0 || g->sw_nnz > (int64_t)INT32_MAX - 2 * C) return arg_error("graph too large for the batched solve");
-    const int32_t nch = (int32_t)((g->sw_nnz + C - 1) / C);
-    const int64_t epad = (int64_t)nch * C;
+    // scratch of the build only: row lengths, padded row offsets, destinations
+    struct Scratch {
+        DevBuf len, row, dst;
+        cudaStream_t s;
+        ~Scratch() {
+            for (DevBuf* b : {&len, &row, &dst}) b->release_on(s);
+        }
+    } t;
+    t.s = s;
     int rc;
+    if ((rc = t.len.grow_on(((size_t)n + 1) * sizeof(uint32_t), s)) ||
+        (rc = t.row.grow_on(((size_t)n + 1) * sizeof(int32_t), s)) ||
+        (rc = t.dst.grow_on((size_t)std::max<int64_t>(g->nnz, 1) * sizeof(int32_t), s)))
+        return rc;
+    k_sp_row_len<<<grid_1d((int64_t)n + 1), 256, 0, s>>>(g->in_row.as<int32_t>(), n, t.len.as<uint32_t>());
+    if ((rc = exclusive_scan_u32(t.len.as<uint32_t>(), t.row.as<uint32_t>(), (int64_t)n + 1, s))) return rc;
+    expand_rows(g->in_row.as<int32_t>(), n, t.dst.as<int32_t>(), s);
+    uint32_t total = 0;
+    if ((rc = cuda_ok(cudaMemcpyAsync(&total, t.row.as<uint32_t>() + n, sizeof(total), cudaMemcpyDeviceToHost, s), "D2H entries")) ||
+        (rc = cuda_ok(cudaStreamSynchronize(s), "SpMM layout")))
+        return rc;
+    const int64_t sw_nnz = total;
+    if (sw_nnz <= 0 || sw_nnz > (int64_t)INT32_MAX - 2 * C) return arg_error("graph too large for the batched solve");
+    const int32_t nch = (int32_t)((sw_nnz + C - 1) / C);
+    const int64_t epad = (int64_t)nch * C;
     if ((rc = w.src.grow_on((size_t)epad * sizeof(int32_t), s)) || (rc = w.c32.grow_on((size_t)epad * sizeof(float), s)) ||
         (rc = w.c64.grow_on((size_t)epad * sizeof(double), s)) || (rc = w.chunks.grow_on((size_t)nch * sizeof(SpChunk), s)))
         return rc;
-    k_sp_entries<<<grid_1d(epad), 256, 0, s>>>(g->sw_col.as<int32_t>(), g->weighted ? g->sw_w.as<float>() : nullptr,
-                                               g->sw_nnz, epad, g->hub_ids.as<int32_t>(), g->nhub,
-                                               g->outw.as<double>(), n, w.src.as<int32_t>(), w.c32.as<float>(),
-                                               w.c64.as<double>());
-    k_sp_marks<<<grid_1d(n), 256, 0, s>>>(g->sw_row.as<int32_t>(), n, w.src.as<int32_t>());
-    k_sp_chunks<<<(nch + 255) / 256, 256, 0, s>>>(g->sw_row.as<int32_t>(), n, (int32_t)g->sw_nnz, C, nch,
+    k_sp_entries<<<grid_1d(g->nnz), 256, 0, s>>>(t.dst.as<int32_t>(), g->in_row.as<int32_t>(), g->in_col.as<int32_t>(),
+                                                 g->weighted ? g->in_w.as<float>() : nullptr, g->nnz,
+                                                 t.row.as<int32_t>(), g->outw.as<double>(), w.src.as<int32_t>(),
+                                                 w.c32.as<float>(), w.c64.as<double>());
+    k_sp_placeholders<<<grid_1d(n), 256, 0, s>>>(g->in_row.as<int32_t>(), t.row.as<int32_t>(), n, sw_nnz, epad,
+                                                 w.src.as<int32_t>(), w.c32.as<float>(), w.c64.as<double>());
+    k_sp_chunks<<<(nch + 255) / 256, 256, 0, s>>>(t.row.as<int32_t>(), n, (int32_t)sw_nnz, C, nch,
                                                   w.chunks.as<SpChunk>());
     if ((rc = cuda_ok(cudaGetLastError(), "SpMM layout"))) return rc;
     w.C = C;
