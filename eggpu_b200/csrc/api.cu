@@ -307,8 +307,37 @@ static int read_states(Plan& plan, int32_t idx, cudaStream_t s, SolveOut* o) {
     return EGPR_SUCC;
 }
 
-// The state of a graph's last single-vector solve (binned or blocked sweep).
+// Enqueues a single-vector solve: the binned sweep (opt-in), the one-kernel solve of
+// a small graph, or the graph's plan.
+static int enqueue_single(egpr_graph* g, double alpha, int32_t max_iter, double tol, bool personalised,
+                          uint32_t flags, cudaStream_t s, int32_t* host_launches) {
+    if (g->bins) return bins_enqueue(g, alpha, max_iter, tol, personalised, flags, s, host_launches);
+    if (!g->small_state.p) return enqueue_plan(g->plan, alpha, max_iter, tol, personalised, flags, s, host_launches);
+    const SmallGraph G{g->n, g->nnz, g->in_row.as<int32_t>(), g->in_col.as<int32_t>(),
+                       g->weighted ? g->in_w.as<float>() : nullptr, g->outw.as<double>(),
+                       personalised ? g->tele.as<float>() : nullptr};
+    float* z = g->z0.as<float>();
+    const SmallWork V{g->small_state.as<SmallState>(), {g->x0.as<float>(), g->x1.as<float>()}, {z, z + g->n},
+                      g->z64.as<double>()};
+    *host_launches = 2;
+    return small_solve(G, V, alpha, tol, max_iter, (flags & EGPR_FLAG_NO_CORRECTION) == 0, g->out.as<double>(), s);
+}
+
+// The state of a graph's last single-vector solve.
 static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
+    if (!g->bins && g->small_state.p) {
+        SmallState st;
+        int rc;
+        if ((rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state")) ||
+            (rc = cuda_ok(cudaStreamSynchronize(s), "solve")))
+            return rc;
+        o->iterations = st.iter;
+        o->converged = st.converged;
+        o->residual = st.residual;
+        o->launches = 0;
+        o->error = st.error;
+        return EGPR_SUCC;
+    }
     if (!g->bins) return read_states(g->plan, 0, s, o);
     return bins_read_state(g, s, &o->iterations, &o->converged, &o->residual, &o->launches, &o->error);
 }
@@ -396,11 +425,7 @@ static int solve_single(egpr_graph* g, double alpha, int32_t max_iter, double to
     {
         NvtxRange nv("egpr solve");
         if ((rc = cuda_ok(cudaEventRecord(g->ev0, s), "event"))) return rc;
-        if (g->bins)
-            rc = bins_enqueue(g, alpha, max_iter, tol, personalised, flags, s, &host_launches);
-        else
-            rc = enqueue_plan(g->plan, alpha, max_iter, tol, personalised, flags, s, &host_launches);
-        if (rc) return rc;
+        if ((rc = enqueue_single(g, alpha, max_iter, tol, personalised, flags, s, &host_launches))) return rc;
         if ((rc = cuda_ok(cudaEventRecord(g->ev1, s), "event"))) return rc;
     }
     NvtxRange nv_read("egpr readback");
@@ -506,7 +531,7 @@ static uint64_t bits_of(double x) {
 int64_t egpr_graph::device_bytes() const {
     int64_t b = 0;
     for (const egpr::DevBuf* d : {&in_row, &in_col, &in_w, &outw, &dangling01, &rank, &idx, &sw_w, &tile_bits, &tile_pair,
-                            &pair_row, &row_step, &steps, &row_tile, &pairs, &scale, &tele, &x0, &x1, &z0, &out, &z64, &plan.d_units,
+                            &pair_row, &row_step, &steps, &row_tile, &pairs, &scale, &tele, &x0, &x1, &z0, &out, &z64, &small_state, &plan.d_units,
                             &plan.d_cta_unit, &plan.d_row_tiles, &plan.d_graphs, &plan.d_states, &plan.d_ndang,
                             &plan.d_ctl, &plan.d_acc})
         b += (int64_t)d->bytes;
@@ -528,7 +553,7 @@ static void destroy_graph_object(egpr_graph* g) {
     g->plan.release();
     for (DevBuf* b : {&g->in_row, &g->in_col, &g->in_w, &g->outw, &g->dangling01, &g->rank, &g->idx, &g->sw_w,
                       &g->tile_bits, &g->tile_pair, &g->pair_row, &g->row_step, &g->steps, &g->row_tile, &g->pairs, &g->scale, &g->tele,
-                      &g->seed_ids, &g->x0, &g->x1, &g->z0, &g->out, &g->z64})
+                      &g->seed_ids, &g->small_state, &g->x0, &g->x1, &g->z0, &g->out, &g->z64})
         b->release();
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
@@ -802,9 +827,12 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
         }
     }
     const size_t nf = (size_t)n * sizeof(float), nd = (size_t)n * sizeof(double);
-    const size_t nz = (size_t)z_stride(g->nsrc);  // by source rank, whole 16-byte units
+    // by source rank, whole 16-byte units; by vertex in the one-kernel solve
+    const bool small = small_wanted(n, g->nnz);
+    const size_t nz = (size_t)std::max<int64_t>(z_stride(g->nsrc), small ? n : 0);
     if ((rc = g->scale.alloc(2 * nf)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
-        (rc = g->z0.alloc(2 * nz * sizeof(float))) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nz * sizeof(double)))) {
+        (rc = g->z0.alloc(2 * nz * sizeof(float))) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nz * sizeof(double))) ||
+        (small && (rc = g->small_state.alloc(sizeof(SmallState))))) {
         destroy_graph_object(g);
         return rc;
     }
@@ -987,11 +1015,7 @@ int egpr_pagerank_enqueue(egpr_graph* g, double alpha, int32_t max_iter, double 
     g->pending_launches = 0;
     if (g->nnz > 0) {
         if ((rc = cuda_ok(cudaEventRecord(g->ev0, g->stream), "event"))) return rc;
-        if (g->bins)
-            rc = bins_enqueue(g, alpha, max_iter, tol, false, flags, g->stream, &g->pending_launches);
-        else
-            rc = enqueue_plan(g->plan, alpha, max_iter, tol, false, flags, g->stream, &g->pending_launches);
-        if (rc) return rc;
+        if ((rc = enqueue_single(g, alpha, max_iter, tol, false, flags, g->stream, &g->pending_launches))) return rc;
         if ((rc = cuda_ok(cudaEventRecord(g->ev1, g->stream), "event"))) return rc;
     }
     g->pending = true;

@@ -247,6 +247,40 @@ struct BinLayout {
     ~BinLayout();
 };
 
+// ---- the one-kernel solve of a small graph (small.cu) ------------------------
+struct SmallState {
+    // residual, dangling mass and rank sum, 2 fixed-point words each; sweep i adds
+    // to set i % 3 while set (i + 1) % 3 is clear
+    unsigned long long acc[3][6];
+    double residual;
+    int32_t iter;
+    int32_t converged;
+    int32_t ndang;
+    uint32_t arrived;           // barrier arrivals of the running kernel
+    int32_t error;
+    int32_t pad;
+    unsigned long long t_begin; // global timer (ns) when the solve's first kernel started
+    unsigned long long t_end;   // global timer (ns) when its last CTA ended
+};
+
+// The inbound CSR (natural source ids) and out-weight sums.
+struct SmallGraph {
+    int32_t n;
+    int64_t nnz;
+    const int32_t* in_row;
+    const int32_t* in_col;
+    const float* in_w;       // NULL = unit weights
+    const double* outw;
+    const float* tele;       // teleport vector, NULL = uniform
+};
+
+struct SmallWork {
+    SmallState* st;
+    float* x[2];             // n each
+    float* z[2];             // n each
+    double* z64;             // n: the correction sweep's carried values (may lie over z)
+};
+
 // ---- prepared graph handle ---------------------------------------------------
 }  // namespace egpr
 
@@ -283,6 +317,7 @@ struct egpr_graph {
     // solve workspace
     egpr::DevBuf scale, tele, x0, x1, z0, out, z64;
     egpr::DevBuf seed_ids;         // seed set of a single-vector PPR solve
+    egpr::DevBuf small_state;      // solves run as one kernel (small.cu) when this is allocated
     egpr::Plan plan;               // single-graph plan
     egpr::SpmmWork* spmm = nullptr; // batched personalised PageRank workspace
     egpr::BinLayout* bins = nullptr; // binned single-graph sweep (null: the tile sweep serves single solves)
@@ -349,6 +384,11 @@ int launch_init(Plan& plan, double alpha, int32_t max_iter, double tol, bool per
                 cudaStream_t stream);
 int launch_loop(Plan& plan, int32_t max_iter, cudaStream_t stream, int32_t* launches);
 int launch_finish(Plan& plan, bool correction, cudaStream_t stream, int32_t* launches);
+
+// The one-kernel solve (small.cu).
+bool small_wanted(int32_t n, int64_t nnz);  // prepared graphs it serves
+int small_solve(const SmallGraph& graph, const SmallWork& work, double alpha, double tol, int32_t max_iter,
+                bool with_correction, double* ranks, cudaStream_t s);
 
 // SpMM personalised PageRank (spmm.cu).  A batched sweep gathers a whole
 // 32-column panel per entry, about seven single-vector sweeps' worth, so

@@ -298,9 +298,9 @@ EGPR_API int egpr_pagerank_csr(const int32_t* V, int32_t len_V, const int32_t* E
  * enqueued on `stream` (a cudaStream_t, NULL = default stream); with stats
  * non-NULL the call waits for it and fills stats (kernel_seconds: device time
  * from the first to the last kernel of the solve, read from the GPU's global
- * timer; n <= 0 zeroes stats).  Every one of the max_iter sweeps is launched:
- * sweeps after convergence return at once but each still costs a kernel
- * launch (a few microseconds), so pick max_iter near the sweeps needed.  The
+ * timer; n <= 0 zeroes stats).  The whole solve is one cooperative kernel, which
+ * ends at the stop rule: a sweep limit far above the sweeps needed costs
+ * nothing, and the launch waits until its CTAs fit the device together.  The
  * array's device address is cached per device for the life of the process;
  * after cudaDeviceReset on that device the cached address is stale, so do not
  * reset a device between calls.
