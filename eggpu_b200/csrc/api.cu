@@ -827,6 +827,7 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
         }
     }
     const size_t nf = (size_t)n * sizeof(float), nd = (size_t)n * sizeof(double);
+    if (g->tune_spmm_chunk == 0) g->tune_spmm_chunk = spmm_chunk_for(g->nnz);
     // by source rank, whole 16-byte units; by vertex in the one-kernel solve
     const bool small = small_wanted(n, g->nnz);
     const size_t nz = (size_t)std::max<int64_t>(z_stride(g->nsrc), small ? n : 0);

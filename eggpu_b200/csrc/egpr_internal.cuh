@@ -312,7 +312,7 @@ struct egpr_graph {
     // layout parameters (egpr_tuning); defaults from the environment
     int32_t tune_cpw = 8;           // sweep: sets the row tile size (row tiles per resident warp)
     int32_t tune_rc = 4;            // sweep: cost of a pair, in entries, when phase 1 is cut into CTA shares
-    int32_t tune_spmm_chunk = 1024; // batched solve: entries per work unit
+    int32_t tune_spmm_chunk = 0;    // batched solve: entries per work unit
     int32_t tuning_recorded = 0;    // the layout came from the persisted tuner choices
     // solve workspace
     egpr::DevBuf scale, tele, x0, x1, z0, out, z64;
@@ -354,7 +354,8 @@ int rebuild_sweep_layout(egpr_graph* g, cudaStream_t s);  // for the graph's cur
 void expand_rows(const int32_t* row, int32_t n, int32_t* dst, cudaStream_t s);
 int default_chunks_per_warp();  // EGPR_CHUNKS_PER_WARP, else 8
 int default_row_cost();         // EGPR_ROW_COST, else 4
-int32_t default_spmm_chunk();   // EGPR_SPMM_CHUNK, else 1024
+int32_t default_spmm_chunk();   // EGPR_SPMM_CHUNK, else 0
+int32_t spmm_chunk_for(int64_t entries);  // the batched solve's tile for a graph of that size
 int export_in_col(const egpr_graph* g, int32_t* host, cudaStream_t s);
 // D2H of a result after the work enqueued on s: a plain async copy into
 // page-locked memory (or under 1 MiB); into pageable memory through the

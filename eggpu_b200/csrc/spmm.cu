@@ -934,14 +934,25 @@ int spmm_grid(bool f64) {
 
 }  // namespace
 
-// Default entries per chunk (a multiple of 32).
+// Entries per chunk when EGPR_SPMM_CHUNK fixes them (a multiple of 32), else 0.
 int32_t default_spmm_chunk() {
     static const int32_t v = [] {
         const char* e = std::getenv("EGPR_SPMM_CHUNK");
-        const int x = e ? std::atoi(e) : 1024;
-        return (x >= 64 && x <= (1 << 16)) ? (x & ~31) : 1024;
+        const int x = e ? std::atoi(e) : 0;
+        return (x >= 64 && x <= (1 << 16)) ? (x & ~31) : 0;
     }();
     return v;
+}
+
+// Entries per chunk for a graph of `entries` inbound entries: about eight chunks of a
+// panel per resident warp, between 128 and 1024 entries.  Fewer chunks leave the last
+// of a launch's few rounds of chunks nearly empty: 45 columns on 1.4 M entries took
+// 1.41 ms with 1024, 1.10 with 512 and 0.95 with 256; a session on 1.9 M entries 23, 19
+// and 16 ms.  With many panels a launch is long and the size matters little (256
+// columns on 16 M entries, 20 sweeps: 65.9, 61.7 and 62.4 ms with 256, 512 and 1024).
+int32_t spmm_chunk_for(int64_t entries) {
+    const int64_t want = entries / ((int64_t)8 * kSpWarps * 148);
+    return want >= 384 ? 1024 : want >= 192 ? 512 : want >= 96 ? 256 : 128;
 }
 
 // Per-graph SpMM workspace: the layout (entry stream and chunks, built on the
