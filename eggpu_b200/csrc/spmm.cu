@@ -945,14 +945,14 @@ int32_t default_spmm_chunk() {
 }
 
 // Entries per chunk for a graph of `entries` inbound entries: about eight chunks of a
-// panel per resident warp, between 128 and 1024 entries.  Fewer chunks leave the last
+// panel per resident warp, between 128 and 512 entries.  Fewer chunks leave the last
 // of a launch's few rounds of chunks nearly empty: 45 columns on 1.4 M entries took
 // 1.41 ms with 1024, 1.10 with 512 and 0.95 with 256; a session on 1.9 M entries 23, 19
 // and 16 ms.  With many panels a launch is long and the size matters little (256
 // columns on 16 M entries, 20 sweeps: 65.9, 61.7 and 62.4 ms with 256, 512 and 1024).
 int32_t spmm_chunk_for(int64_t entries) {
     const int64_t want = entries / ((int64_t)8 * kSpWarps * 148);
-    return want >= 384 ? 1024 : want >= 192 ? 512 : want >= 96 ? 256 : 128;
+    return want >= 384 ? 512 : want >= 192 ? 512 : want >= 96 ? 256 : 128;
 }
 
 // Per-graph SpMM workspace: the layout (entry stream and chunks, built on the
@@ -964,7 +964,8 @@ struct SpmmWork {
     int64_t epad = 0;
     DevBuf src, c32, c64, chunks;
     int32_t cap_panels = 0;
-    DevBuf X0, X1, out64, cols, parts, span_cnt, gacc, colsum, ctl, meta, params, out, tele, tele_v;
+    DevBuf X0, X1, out64, cols, parts, span_cnt, gacc, colsum, ctl, meta, params, out, out_b, states, tele, tele_v;
+    cudaStream_t copy = nullptr;  // results of one group travel here while the next one is solved
     cudaGraph_t cg = nullptr;
     cudaGraphExec_t cg_exec = nullptr;
     cudaGraphConditionalHandle cond = 0;
@@ -974,15 +975,16 @@ struct SpmmWork {
         if (cg_exec) cudaGraphExecDestroy(cg_exec);
         if (cg) cudaGraphDestroy(cg);
         for (DevBuf* b : buffers()) b->release();
+        if (copy) cudaStreamDestroy(copy);
     }
     // Frees the buffers in the order of stream s (no wait for the device, so
     // other graphs' solves on other streams keep running).
     void release_on(cudaStream_t s) {
         for (DevBuf* b : buffers()) b->release_on(s);
     }
-    std::array<DevBuf*, 18> buffers() {
+    std::array<DevBuf*, 20> buffers() {
         return {&src, &c32, &c64, &chunks, &X0, &X1, &out64, &cols, &parts, &span_cnt, &gacc, &colsum, &ctl,
-                &meta, &params, &out, &tele, &tele_v};
+                &meta, &params, &out, &out_b, &states, &tele, &tele_v};
     }
 };
 
@@ -1124,10 +1126,12 @@ void build_loop_graph(SpmmWork& w, int grid) {
 
 using ColEntries = std::vector<std::pair<int32_t, float>>;
 
-// One device solve over columns [j0, j0 + kg) (kg <= kMaxPanels * 32).
-int solve_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, double tol, int32_t j0, int32_t kg,
-                const std::vector<ColEntries>& per_col, uint32_t flags, double* out, egpr_stats* stats) {
-    const double t0 = wall_seconds();
+// One device solve over columns [j0, j0 + kg) (kg <= kMaxPanels * 32), enqueued on the
+// graph's stream between events e0 and e1: results to `out`, the column states and
+// the control block behind them to `states`.
+int enqueue_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, double tol, int32_t j0, int32_t kg,
+                  const std::vector<ColEntries>& per_col, uint32_t flags, double* out, unsigned char* states,
+                  cudaEvent_t e0, cudaEvent_t e1, int32_t* host_launches) {
     const int32_t n = g->n;
     cudaStream_t s = g->stream;
     const int32_t npanels = (kg + kLanes - 1) / kLanes;
@@ -1147,8 +1151,7 @@ int solve_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, doub
     for (int32_t jj = 0; jj < kg; ++jj)
         for (const auto& pr : per_col[(size_t)(j0 + jj)]) tt[(size_t)tidx[(size_t)pr.first] * ld + jj] = pr.second;
     if ((rc = w.tele.grow_on(tt.size() * sizeof(float), s)) ||
-        (rc = w.tele_v.grow_on((size_t)std::max(nt, 1) * sizeof(int32_t), s)) ||
-        (rc = w.out.grow_on((size_t)kg * n * sizeof(double), s)))
+        (rc = w.tele_v.grow_on((size_t)std::max(nt, 1) * sizeof(int32_t), s)))
         return rc;
     if ((rc = cuda_ok(cudaMemcpyAsync(w.tele.p, tt.data(), tt.size() * sizeof(float), cudaMemcpyHostToDevice, s),
                       "H2D teleport")) ||
@@ -1194,7 +1197,7 @@ int solve_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, doub
     const int64_t work = 4 * (int64_t)npanels * w.epad;
     const int grid = work_grid(work, spmm_grid(false));
     const int grid64 = work_grid(work, spmm_grid(true));
-    if ((rc = cuda_ok(cudaEventRecord(g->ev0, s), "event"))) return rc;
+    if ((rc = cuda_ok(cudaEventRecord(e0, s), "event"))) return rc;
     k_sp_meta<<<grid_1d(n), 256, 0, s>>>(g->outw.as<double>(), n, w.meta.as<uint32_t>());
     if (nt > 0) k_sp_tele_rows<<<(nt + 255) / 256, 256, 0, s>>>(w.tele_v.as<int32_t>(), nt, w.meta.as<uint32_t>());
     k_sp_init<<<dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 1) * 8 / 256 + 1, 148 * 8)),
@@ -1227,41 +1230,31 @@ int solve_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, doub
     {
         dim3 gr((unsigned)((n + kNormRows - 1) / kNormRows), (unsigned)npanels);
         k_sp_normalize<<<gr, 256, 0, s>>>(w.out64.as<double>(), w.X0.as<float>(), w.X1.as<float>(),
-                                          w.cols.as<ColState>(), n, kg, correction ? 0 : 1, w.out.as<double>(),
-                                          nullptr);
+                                          w.cols.as<ColState>(), n, kg, correction ? 0 : 1, out, nullptr);
         launches += 1;
     }
-    if ((rc = cuda_ok(cudaGetLastError(), "spmm finish"))) return rc;
-    if ((rc = cuda_ok(cudaEventRecord(g->ev1, s), "event"))) return rc;
-    // out == NULL: device timing only (the tuner)
-    if (out && (rc = download_d2h(out, w.out.p, (size_t)kg * n * sizeof(double), s, "D2H ranks"))) return rc;
-    std::vector<ColState> hc((size_t)npanels * kLanes);
-    Ctl ctl;
-    if ((rc = cuda_ok(cudaMemcpyAsync(hc.data(), w.cols.p, hc.size() * sizeof(ColState), cudaMemcpyDeviceToHost, s),
-                      "D2H cols")) ||
-        (rc = cuda_ok(cudaMemcpyAsync(&ctl, w.ctl.p, sizeof(ctl), cudaMemcpyDeviceToHost, s), "D2H ctl")) ||
-        (rc = cuda_ok(cudaStreamSynchronize(s), "batch solve")))
+    if ((rc = cuda_ok(cudaGetLastError(), "spmm finish")) || (rc = cuda_ok(cudaEventRecord(e1, s), "event")) ||
+        (rc = cuda_ok(cudaMemcpyAsync(states, w.cols.p, (size_t)npanels * kLanes * sizeof(ColState),
+                                      cudaMemcpyDeviceToDevice, s), "column states")) ||
+        (rc = cuda_ok(cudaMemcpyAsync(states + (size_t)npanels * kLanes * sizeof(ColState), w.ctl.p, sizeof(Ctl),
+                                      cudaMemcpyDeviceToDevice, s), "column states")))
         return rc;
-    if (ctl.error) return ctl.error;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
-    if (stats) {
-        // compulsory bytes of one sweep: per panel the entry stream, the
-        // previous and the next iterate, and the row meta
-        const int64_t bytes = (int64_t)npanels * (w.epad * 8 + 2 * ((int64_t)n + 1) * kLanes * 4 + 4 * (int64_t)n);
-        for (int32_t jj = 0; jj < kg; ++jj) {
-            egpr_stats& st = stats[jj];
-            st.iterations = hc[(size_t)jj].iter;
-            st.converged = hc[(size_t)jj].converged;
-            st.residual = hc[(size_t)jj].residual;
-            st.kernel_seconds = ms * 1e-3;
-            st.total_seconds = wall_seconds() - t0;
-            st.bytes_per_iter = bytes;
-            st.launches = launches + ctl.launches;
-            st.reserved = 0;
-        }
-    }
+    *host_launches = launches;
     return EGPR_SUCC;
+}
+
+// Columns solved together.  A large graph's panels keep the GPU busy few at a time
+// (a panel sweep of 4 M entries takes about 0.1 ms), and a panel's results take as long
+// to copy out as many of its sweeps: there a group is three panels, whose results
+// travel while the next group is solved.  R-MAT scale 20, k = 256, 20 sweeps, 2.1 GB of
+// results: 104 ms in one group, 93.8, 83.4, 79.8 and 85.3 ms in groups of one to four
+// panels (fewer panels per launch fill the GPU less well, more leave more to copy at
+// the end).  Smaller graphs need many panels per launch and have little to copy.
+int32_t group_columns(const egpr_graph* g, const SpmmWork& w, int32_t k) {
+    constexpr int64_t kPanelEntries = 4 << 20;
+    constexpr int32_t kGroupPanels = 3;
+    const bool large = w.epad >= kPanelEntries && (int64_t)g->n * kLanes * (int64_t)sizeof(double) >= (int64_t)16 << 20;
+    return std::min(k, (large ? kGroupPanels : kMaxPanels) * kLanes);
 }
 
 }  // namespace
@@ -1314,22 +1307,84 @@ int ppr_batch_solve(egpr_graph* g, double alpha, int32_t max_iter, double tol, i
     SpmmWork& w = *g->spmm;
     cudaStream_t s = g->stream;
     if (!w.C && (rc = build_spmm_layout(g, w, s))) return rc;
-    // device solves of up to kMaxPanels panels each
-    constexpr int32_t kGroup = kMaxPanels * kLanes;
-    for (int32_t j0 = 0; j0 < k; j0 += kGroup) {
-        const int32_t kg = std::min(kGroup, k - j0);
-        if ((rc = solve_group(g, w, alpha, max_iter, tol, j0, kg, per_col, flags, out ? out + (size_t)j0 * n : nullptr,
-                              stats ? stats + j0 : nullptr)))
+    // Groups of columns: the results of a group are copied out (on a stream of their
+    // own, from one of two buffers) while the next group is solved.
+    const int32_t group = group_columns(g, w, k), ngroups = (k + group - 1) / group;
+    struct Events {
+        std::vector<cudaEvent_t> ev;
+        ~Events() {
+            for (cudaEvent_t e : ev)
+                if (e) cudaEventDestroy(e);
+        }
+    } E;
+    E.ev.assign((size_t)3 * ngroups, nullptr);  // per group: begin, end, results copied
+    for (size_t i = 0; i < E.ev.size(); ++i)
+        if ((rc = cuda_ok(i % 3 == 2 ? cudaEventCreateWithFlags(&E.ev[i], cudaEventDisableTiming) : cudaEventCreate(&E.ev[i]), "event")))
             return rc;
+    if (!w.copy && (rc = cuda_ok(cudaStreamCreateWithFlags(&w.copy, cudaStreamNonBlocking), "stream"))) return rc;
+    const size_t state_bytes = (size_t)((group + kLanes - 1) / kLanes) * kLanes * sizeof(ColState) + sizeof(Ctl);
+    const size_t state_stride = (state_bytes + 255) & ~(size_t)255;
+    if ((rc = w.states.grow_on(state_stride * (size_t)ngroups, s)) ||
+        (rc = w.out.grow_on((size_t)group * n * sizeof(double), s)) ||
+        (ngroups > 1 && (rc = w.out_b.grow_on((size_t)group * n * sizeof(double), s))))
+        return rc;
+    std::vector<int32_t> launches((size_t)ngroups, 0);
+    auto columns = [&](int32_t i) { return std::min(group, k - i * group); };
+    auto copy_out = [&](int32_t i) {
+        if (!out) return (int)EGPR_SUCC;  // device timing only (the tuner)
+        int r = cuda_ok(cudaStreamWaitEvent(w.copy, E.ev[(size_t)3 * i + 1], 0), "event");
+        if (!r)
+            r = download_d2h(out + (size_t)i * group * n, (i & 1 ? w.out_b : w.out).p, (size_t)columns(i) * n * sizeof(double),
+                             w.copy, "D2H ranks");
+        return r ? r : cuda_ok(cudaEventRecord(E.ev[(size_t)3 * i + 2], w.copy), "event");
+    };
+    rc = EGPR_SUCC;
+    for (int32_t i = 0; i < ngroups && !rc; ++i) {
+        // group i writes the buffer that group i - 2 is copied from
+        if (i >= 2 && out) rc = cuda_ok(cudaStreamWaitEvent(s, E.ev[(size_t)3 * (i - 2) + 2], 0), "event");
+        if (!rc)
+            rc = enqueue_group(g, w, alpha, max_iter, tol, i * group, columns(i), per_col, flags,
+                               (i & 1 ? w.out_b : w.out).as<double>(), w.states.as<unsigned char>() + (size_t)i * state_stride,
+                               E.ev[(size_t)3 * i], E.ev[(size_t)3 * i + 1], &launches[(size_t)i]);
+        if (!rc && i > 0) rc = copy_out(i - 1);
     }
-    if (stats && k > kGroup) {  // the whole batch's device time in every column
-        double ks = 0.0;
-        for (int32_t j0 = 0; j0 < k; j0 += kGroup) ks += stats[j0].kernel_seconds;
-        for (int32_t j = 0; j < k; ++j) {
-            stats[j].kernel_seconds = ks;
-            stats[j].total_seconds = wall_seconds() - t0;
+    if (!rc) rc = copy_out(ngroups - 1);
+    std::vector<unsigned char> hs(state_stride * (size_t)ngroups);
+    if (!rc) rc = cuda_ok(cudaMemcpyAsync(hs.data(), w.states.p, hs.size(), cudaMemcpyDeviceToHost, s), "D2H states");
+    // nothing may be in flight into the caller's memory or from the buffers on return
+    const int rc_s = cuda_ok(cudaStreamSynchronize(s), "batch solve");
+    const int rc_c = cuda_ok(cudaStreamSynchronize(w.copy), "batch results");
+    if (rc || (rc = rc_s) || (rc = rc_c)) return rc;
+    double kernel_s = 0.0;
+    for (int32_t i = 0; i < ngroups; ++i) {
+        const int32_t npanels = (columns(i) + kLanes - 1) / kLanes;
+        Ctl ctl;
+        std::memcpy(&ctl, hs.data() + (size_t)i * state_stride + (size_t)npanels * kLanes * sizeof(ColState), sizeof(ctl));
+        if (ctl.error) return ctl.error;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, E.ev[(size_t)3 * i], E.ev[(size_t)3 * i + 1]);
+        kernel_s += ms * 1e-3;
+        if (!stats) continue;
+        // compulsory bytes of one sweep: per panel the entry stream, the previous
+        // and the next iterate, and the row meta
+        const int64_t bytes = (int64_t)npanels * (w.epad * 8 + 2 * ((int64_t)n + 1) * kLanes * 4 + 4 * (int64_t)n);
+        for (int32_t jj = 0; jj < columns(i); ++jj) {
+            ColState cs;
+            std::memcpy(&cs, hs.data() + (size_t)i * state_stride + (size_t)jj * sizeof(ColState), sizeof(cs));
+            egpr_stats& st = stats[(size_t)i * group + jj];
+            st.iterations = cs.iter;
+            st.converged = cs.converged;
+            st.residual = cs.residual;
+            st.bytes_per_iter = bytes;
+            st.launches = launches[(size_t)i] + ctl.launches;
+            st.reserved = 0;
         }
     }
+    if (stats)  // the whole batch's device time in every column
+        for (int32_t j = 0; j < k; ++j) {
+            stats[j].kernel_seconds = kernel_s;
+            stats[j].total_seconds = wall_seconds() - t0;
+        }
     return EGPR_SUCC;
 }
 
