@@ -378,8 +378,8 @@ def measure_workload(name, args, rank, world, local, dist, sweeps, with_e2e=True
                               else "egpr_graph_autotune before timing"}},
         "hbm_gbs": bytes_per_iter * sweeps / t_step / 1e9,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": profile_traffic(f"k_sweep_{name}.md"),
-                     "kernel": "k_sweep<float> (fused sweep)", "peak_source": peak_kind,
+                     "traffic": profile_traffic(f"sweep_phases_{name}.md"),
+                     "kernel": "k_gather<float> + k_rows<float> (one sweep)", "peak_source": peak_kind,
                      "bytes_per_launch": bytes_per_iter, "launch_ms": t_sweep * 1e3,
                      "timing": "CUDA events on the launch stream; per-sweep time = (T(2S) - T(S)) / S"},
         "gpu_launches": int(st["launches"] * args.steps + st2["launches"] * max(1, args.steps // 2)),

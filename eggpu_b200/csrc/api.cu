@@ -302,7 +302,7 @@ static int read_states(Plan& plan, int32_t idx, cudaStream_t s, SolveOut* o) {
     o->iterations = st.iter;
     o->converged = st.converged;
     o->residual = st.residual;
-    o->launches = ctl.launches;
+    o->launches = 2 * ctl.launches;  // two phases per sweep
     o->error = ctl.error;
     return EGPR_SUCC;
 }
@@ -695,7 +695,7 @@ bool tuning_valid(const egpr_tuning& t) {
 }
 
 // Rebuilds the sweep layout and the single-graph plan for the graph's current
-// parameters (the inbound CSR and the hub codes stay as prepared).
+// parameters (the inbound CSR and the ranking stay as prepared).
 int rebuild_sweep(egpr_graph* g) {
     cudaStream_t s = g->own_stream;
     int rc;
@@ -1146,7 +1146,7 @@ int egpr_pagerank_multi(int32_t count, egpr_graph* const* graphs, double alpha, 
             o.iterations = st[i].iter;
             o.converged = st[i].converged;
             o.residual = st[i].residual;
-            fill_stats(&stats[live_idx[i]], live[i], o, ms * 1e-3, total, host_launches + ctl.launches);
+            fill_stats(&stats[live_idx[i]], live[i], o, ms * 1e-3, total, host_launches + 2 * ctl.launches);
         }
     }
     return EGPR_SUCC;

@@ -320,7 +320,7 @@ struct egpr_graph {
     egpr::DevBuf small_state;      // solves run as one kernel (small.cu) when this is allocated
     egpr::Plan plan;               // single-graph plan
     egpr::SpmmWork* spmm = nullptr; // batched personalised PageRank workspace
-    egpr::BinLayout* bins = nullptr; // binned single-graph sweep (null: the tile sweep serves single solves)
+    egpr::BinLayout* bins = nullptr; // binned single-graph sweep (null: the other paths serve single solves)
     int32_t sessions = 0;            // live batched-solve sessions (egpr_session_*) on this graph
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr; // active stream (own or user-given)

@@ -10,7 +10,7 @@
 //
 // Layout, built once per graph and kept with it:
 //   * the entry stream: the inbound CSR in row order with one placeholder in
-//     every empty row (the sweep's padded CSR), padded with placeholders to a
+//     every empty row, padded with placeholders to a
 //     whole number of chunks.  Per entry the source vertex, with bit 31 set on
 //     the last entry of each row (placeholders read the all-zero row n), and
 //     the coefficient w / outw[source] in FP32 and in FP64 (0 for placeholders

@@ -106,8 +106,8 @@ EGPR_API const char* egpr_last_error(void);
 /*
  * Uploads an out-edge CSR and prepares it on the current device: FP64
  * out-weight sums, inbound CSR with entries in ascending source order,
- * dangling mask, and the sweep's layout (rows padded to end on an entry of
- * their own, 256-entry warp tiles, cost-balanced chunks).  Replaces the host-side
+ * dangling mask, and the sweep's layout (entries by block of sources and
+ * row, 256-entry warp tiles, row tiles of equal cost).  Replaces the host-side
  * build_inbound_from_csr + H2D of pagerank.cu:286-347,472-518, done on the
  * GPU.  V[n+1] must be non-decreasing with V[0]==0 and V[n]==m (the CSR the
  * reference's gen_CSR / load_csr_files produce); destinations outside [0,n)
@@ -142,8 +142,9 @@ EGPR_API int egpr_graph_set_stream(egpr_graph* g, void* stream);
  * shapes (pagerank.cu), so nothing there is tuned per graph.
  */
 typedef struct egpr_tuning {
-    int32_t chunks_per_warp; /* single-vector sweep: work-queue chunks per resident warp */
-    int32_t row_cost;        /* single-vector sweep: cost of finishing a row, in entries, when cutting chunks */
+    int32_t chunks_per_warp; /* single-vector sweep: row tiles per resident CTA of its second phase, in quarters */
+    int32_t row_cost;        /* single-vector sweep: cost of a (block, row) sum, in entries, when its first phase is
+                                cut into CTA shares */
     int32_t spmm_chunk;      /* batched solve: inbound entries per work unit (the tile along the entries) */
     int32_t configs_tried;   /* egpr_graph_autotune: layouts measured */
     double sweep_ms;         /* egpr_graph_autotune: per-sweep device time of the chosen sweep layout */
