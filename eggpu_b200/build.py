@@ -79,7 +79,7 @@ def _flags_changed(key: str, flags) -> bool:
 def build_engine(verbose: bool = False, ptxas_info: bool = False, force: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
     nvcc = _nvcc()
-    headers = list(CSRC.glob("*.cuh")) + [ROOT / "include" / "egpr.h"]
+    headers = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), ROOT / "include" / "egpr.h"]
     all_new = _forced(force) | _flags_changed("libegpr", [*ARCH, *NVCC_FLAGS])
     objs = []
     for src in CUDA_SOURCES:

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/egpr.h"
+#include "sweep_cut.h"
 
 namespace egpr {
 
@@ -52,6 +53,7 @@ constexpr int kBlockBits = 15;     // bits of an index inside a block (kBlockSrc
 // chunk (a longer one becomes several pairs), so chunks are independent.
 constexpr int kLaneItems = 8;
 constexpr int kTileItems = 32 * kLaneItems;
+static_assert(kTileItems == kCutTileEntries, "the cutting counts the layout's tiles");
 // Per tile and lane one 16-bit word: the lane's run-end marks (low byte) and the
 // number of marks in the lanes below it (high byte); 64 bytes per tile.
 constexpr int kTileWords = 16;
@@ -87,13 +89,6 @@ struct GraphDev {
     int32_t nsrc;            // ranked sources
     int32_t nblocks;
     int32_t chunk_shift;
-};
-
-// A CTA's piece of phase 1: tiles [tile0, tile1) of one block of one graph.
-struct GatherUnit {
-    int32_t graph;
-    int32_t block;
-    int32_t tile0, tile1;
 };
 
 struct GraphState {

@@ -843,7 +843,7 @@ int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_
     std::vector<int32_t> ndang((size_t)count);
     int32_t max_n = 0, max_rows = kRowGroup;
     int64_t entries = 0, nrt = 0;
-    double cost = 0.0;  // of phase 1: entries + the graph's pair cost per pair
+    std::vector<CutGraph> cuts((size_t)count);
     for (int32_t gi = 0; gi < count; ++gi) {
         const egpr_graph* g = graphs[gi];
         views[(size_t)gi] = graph_dev_view(g);
@@ -852,7 +852,7 @@ int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_
         entries += g->nnz;
         nrt += g->nrow_tiles;
         max_rows = std::max(max_rows, g->max_tile_rows);
-        cost += (double)g->h_block_tile.back() * kTileItems + (double)g->tune_rc * g->h_block_pair.back();
+        cuts[(size_t)gi] = CutGraph{g->h_block_tile.data(), g->h_block_pair.data(), g->nblocks, g->chunk_shift, g->tune_rc};
     }
     if (nrt > INT32_MAX / 2) return EGPR_UNSUPPORTED_GRAPH;
     plan.ngraphs = count;
@@ -860,39 +860,11 @@ int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_
     plan.max_rows = max_rows;
     plan.nrow_tiles = (int32_t)nrt;
     plan.grid = work_grid(entries, sweep_grid());
-    // phase 1: equal shares of the cost, contiguous in (graph, block, tile)
+    // phase 1
     std::vector<GatherUnit> units;
-    std::vector<int32_t> cta_unit(1, 0);
-    {
-        const double share = cost / plan.grid;
-        double used = 0.0;  // of the current CTA's share
-        for (int32_t gi = 0; gi < count; ++gi) {
-            const egpr_graph* g = graphs[gi];
-            for (int32_t b = 0; b < g->nblocks; ++b) {
-                const int32_t t1 = g->h_block_tile[(size_t)b + 1];
-                int32_t t = g->h_block_tile[(size_t)b];
-                const double per_tile = kTileItems + (double)g->tune_rc *
-                                        (g->h_block_pair[(size_t)b + 1] - g->h_block_pair[(size_t)b]) / std::max(1, t1 - t);
-                while (t < t1) {
-                    const bool last = (int32_t)cta_unit.size() >= plan.grid;  // the last CTA takes the rest
-                    if (!last && used >= share) {
-                        cta_unit.push_back((int32_t)units.size());
-                        used = 0.0;
-                        continue;
-                    }
-                    int64_t take = last ? t1 - t : (int64_t)((share - used) / per_tile + 0.999);
-                    // whole chunks
-                    take = ((take + ((int64_t)1 << g->chunk_shift) - 1) >> g->chunk_shift) << g->chunk_shift;
-                    take = std::max<int64_t>(1, std::min<int64_t>(take, t1 - t));
-                    units.push_back(GatherUnit{gi, b, t, t + (int32_t)take});
-                    used += per_tile * (double)take;
-                    t += (int32_t)take;
-                }
-            }
-        }
-        while ((int32_t)cta_unit.size() <= plan.grid) cta_unit.push_back((int32_t)units.size());
-        if (units.empty()) units.push_back(GatherUnit{0, 0, 0, 0});
-    }
+    std::vector<int32_t> cta_unit;
+    cut_gather_units(cuts.data(), count, plan.grid, units, cta_unit);
+    if (units.empty()) units.push_back(GatherUnit{0, 0, 0, 0});
     // phase 2: row tiles in row order (their costs are about equal)
     std::vector<int2> order;
     order.reserve((size_t)std::max<int64_t>(nrt, 1));

@@ -82,11 +82,40 @@ def test_one_source_with_every_entry_and_empty_rows(layout, n):
     _check(V, E, W)
 
 
-def test_long_runs_cross_chunks(layout):
-    # 8 M entries: chunks of four tiles; a few rows hold most of a block's entries
-    n, m = 30011, 8_000_000
-    rng = np.random.default_rng(5)
+CHUNKED = 2 * 32 * 1024  # entries per SM from which chunks have four tiles: two of them for each of 32 warps
+
+
+def _long_runs(n, m, seed, weighted):
+    """A few rows hold most of a block's entries."""
+    rng = np.random.default_rng(seed)
     src = np.concatenate([np.arange(n), rng.integers(0, n, m)])
     dst = np.concatenate([(np.arange(n) + 1) % n, np.where(rng.random(m) < 0.7, rng.integers(0, 5, m), rng.integers(0, n, m))])
-    V, E, W = _csr(n, src, dst, True, 6)
+    return _csr(n, src, dst, weighted, seed + 1)
+
+
+def test_long_runs_cross_chunks():
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    V, E, W = _long_runs(30011, CHUNKED * sms, 5, True)
+    assert len(E) >= CHUNKED * sms
     _check(V, E, W, sweeps=3)
+
+
+def test_every_cut_of_a_chunked_plan_gives_the_same_bits():
+    """Row sums are order-free and runs end at fixed chunks, so the cuts between the CTAs
+    of the first phase change nothing; one graph per solve and two in one plan."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    graphs = [_native.PreparedGraph(*_long_runs(n, CHUNKED * sms + n, n, False)) for n in (70001, 30011)]
+    o = {"max_iter": 3, "tol": 0.0}
+    first = [pg.pagerank(**o)[0] for pg in graphs]
+    for row_cost in (0, 1, 2, 3, 5, 7, 8, 13, 33, 64):
+        for pg, want in zip(graphs, first):
+            pg.set_tuning(row_cost=row_cost)
+            assert np.array_equal(pg.pagerank(**o)[0], want), row_cost
+        outs, _ = _native.pagerank_multi(graphs, **o)
+        assert all(np.array_equal(a, b) for a, b in zip(outs, first)), row_cost
+    for pg in graphs:
+        pg.close()
