@@ -219,24 +219,22 @@ void DevBuf::release_on(cudaStream_t s) {
 
 Plan::~Plan() { release(); }
 
+void Plan::release_loops() {
+    for (Loop& l : loops) {
+        if (l.exec) cudaGraphExecDestroy(l.exec);
+        if (l.graph) cudaGraphDestroy(l.graph);
+        l = Loop();
+    }
+}
+
 void Plan::release() {
-    if (cg_exec) cudaGraphExecDestroy(cg_exec);
-    if (cg) cudaGraphDestroy(cg);
-    cg_exec = nullptr;
-    cg = nullptr;
-    cond = 0;
-    cg_failed = false;
+    release_loops();
     for (DevBuf* b : {&d_units, &d_cta_unit, &d_row_tiles, &d_graphs, &d_states, &d_ndang, &d_ctl, &d_acc}) b->release();
     ngraphs = grid = row_grid = nrow_tiles = max_rows = max_n = nacc = 0;
 }
 
 void Plan::release_on(cudaStream_t s) {
-    if (cg_exec) cudaGraphExecDestroy(cg_exec);
-    if (cg) cudaGraphDestroy(cg);
-    cg_exec = nullptr;
-    cg = nullptr;
-    cond = 0;
-    cg_failed = false;
+    release_loops();
     for (DevBuf* b : {&d_units, &d_cta_unit, &d_row_tiles, &d_graphs, &d_states, &d_ndang, &d_ctl, &d_acc})
         b->release_on(s);
     ngraphs = grid = row_grid = nrow_tiles = max_rows = max_n = nacc = 0;
@@ -285,8 +283,9 @@ static int enqueue_plan(Plan& plan, double alpha, int32_t max_iter, double tol, 
     int rc;
     if ((rc = launch_init(plan, alpha, max_iter, tol, personalised, s))) return rc;
     int32_t l_loop = 0, l_fin = 0;
-    if ((rc = launch_loop(plan, max_iter, s, &l_loop))) return rc;
-    if ((rc = launch_finish(plan, (flags & EGPR_FLAG_NO_CORRECTION) == 0, s, &l_fin))) return rc;
+    const bool watch = rows_need_watch(plan, alpha, personalised);
+    if ((rc = launch_loop(plan, max_iter, watch, s, &l_loop))) return rc;
+    if ((rc = launch_finish(plan, (flags & EGPR_FLAG_NO_CORRECTION) == 0, watch, s, &l_fin))) return rc;
     *host_launches = 3 + l_fin;  // init kernels + finish kernels; sweeps are counted on the device
     return EGPR_SUCC;
 }

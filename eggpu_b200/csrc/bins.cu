@@ -484,7 +484,6 @@ __global__ void k_bins_state(GraphState* st, Ctl* ctl, int32_t n, int32_t ndang,
     s.max_iter = max_iter;
     s.done = 0;
     s.converged = 0;
-    s.fx_unit = 0.f;  // the tile sweep's
     s.personalised = personalised;
     *st = s;
     Ctl c;

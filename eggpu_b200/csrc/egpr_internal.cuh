@@ -105,7 +105,6 @@ struct GraphState {
     int32_t max_iter;
     int32_t done;
     int32_t converged;
-    float fx_unit;     // phase 2 adds in units of 1 / fx_unit (a power of two)
     int32_t personalised;  // teleport from GraphDev::tele instead of 1/n
 };
 
@@ -166,11 +165,14 @@ struct Plan {
     int32_t max_n = 0;
     DevBuf d_units, d_cta_unit, d_row_tiles, d_graphs, d_states, d_ndang, d_ctl, d_acc;
     int32_t nacc = 0;                 // accumulator slots
-    cudaGraph_t cg = nullptr;
-    cudaGraphExec_t cg_exec = nullptr;
-    cudaGraphConditionalHandle cond = 0;
-    bool cg_failed = false;
+    // the sweeps as a CUDA graph, without and with the watch for small row sums (sweep.cu)
+    struct Loop {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        bool failed = false;
+    } loops[2];
     ~Plan();
+    void release_loops();
     void release();
     void release_on(cudaStream_t s);  // buffers used by stream s only: freed in its order
 };
@@ -374,12 +376,13 @@ int sweep_resident_warps();
 int work_grid(int64_t entries, int full);  // CTAs of a launch over that many entries
 int64_t z_stride(int32_t nsrc);    // values per parity of z (whole 16-byte units past the last block)
 int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_t stream);
-int plan_capture_loop(Plan& plan, cudaStream_t stream);
 GraphDev graph_dev_view(const egpr_graph* g);
 int launch_init(Plan& plan, double alpha, int32_t max_iter, double tol, bool personalised,
                 cudaStream_t stream);
-int launch_loop(Plan& plan, int32_t max_iter, cudaStream_t stream, int32_t* launches);
-int launch_finish(Plan& plan, bool correction, cudaStream_t stream, int32_t* launches);
+// Whether rows of a solve may get nothing but their sum: then phase 2 watches for small sums.
+bool rows_need_watch(const Plan& plan, double alpha, bool personalised);
+int launch_loop(Plan& plan, int32_t max_iter, bool watch, cudaStream_t stream, int32_t* launches);
+int launch_finish(Plan& plan, bool correction, bool watch, cudaStream_t stream, int32_t* launches);
 
 // The one-kernel solve (small.cu).
 bool small_wanted(int32_t n, int64_t nnz);  // prepared graphs it serves

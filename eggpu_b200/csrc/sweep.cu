@@ -123,7 +123,6 @@ struct RowView {
     double jump;            // (1-alpha)/n + dangling term (uniform teleport)
     double dmass;           // dangling term alone (personalised teleport)
     double one_minus_alpha;
-    float unit;             // fixed-point units per 1 of a row's sum
     int32_t personalised;
 };
 
@@ -132,7 +131,6 @@ __device__ RowView make_view(const GraphDev& G, GraphState* st, int32_t iter) {
     RowView W;
     W.one_minus_alpha = 1.0 - st->alpha;
     W.personalised = st->personalised;
-    W.unit = st->fx_unit;
     W.rowd = G.rowd;
     W.tele = G.tele;
     W.out = G.out;
@@ -434,13 +432,28 @@ __global__ void __launch_bounds__(32 * kGatherWarps<Real>, 1) k_gather(SweepPara
 }
 
 // ---- phase 2: pairs to rows ---------------------------------------------------------
-// A row's sum is a 64-bit two's-complement integer in units of 1 / W.unit (2^-62
-// for alpha in [0, 1]: sums stay below 1, and the smallest row value of a graph of
-// 2^25 vertices keeps 34 bits, more than FP32's 24).  It is held as two words, added
+// A row's sum is a 64-bit integer in units of 2^-62 (alpha lies in [0, 1] here and ranks
+// sum to 1, so a row's sum stays below 2).  It is held as two words, added
 // with native 32-bit shared-memory atomics and a carry (4 to 6 per clock per SM
 // measured; a 64-bit shared atomicAdd is a compare-and-swap loop, 2 to 5).  The FP64
 // sweep adds what is left below the unit in a second such integer, in units 2^-44
 // smaller: 106 bits.
+//
+// A sum of at least 2^-36 (FP64: 2^-50) keeps 26 (56) bits, and so does every pair of that
+// size: less error than a chain of FP32 (FP64) adds has.  Smaller sums lose bits; they
+// matter only where a row gets nothing else, that is in a personalised solve on a
+// graph without dangling mass, far from the seeds.  There row tiles with smaller pairs
+// add their smallest rows again in finer units (refine_rows).
+constexpr double kUnit = 4611686018427387904.0;    // 2^62 units per 1
+constexpr int kFineShift = 36;                     // log2 between one unit and the next finer
+constexpr double kFine = 68719476736.0;            // 2^36
+template <typename Real>
+constexpr int kRowBits = std::is_same<Real, double>::value ? 12 : 26;  // log2 of the units a sum has at least
+template <typename Real>
+constexpr int kFineLevels = std::is_same<Real, double>::value ? 4 : 3;  // FP32: to its smallest number, 2^-149
+// A term of every row of at least this much makes the bits below the unit immaterial.
+template <typename Real>
+constexpr double kRowFloor = std::is_same<Real, double>::value ? 1.0 / 4503599627370496.0 : 1.0 / 274877906944.0;  // 2^-52, 2^-38
 __device__ __forceinline__ void add_word(uint32_t* lo, uint32_t* hi, unsigned long long q) {
     const uint32_t ql = (uint32_t)q;
     uint32_t qh = (uint32_t)(q >> 32);
@@ -451,6 +464,9 @@ __device__ __forceinline__ void add_word(uint32_t* lo, uint32_t* hi, unsigned lo
     if (qh) atomicAdd(hi, qh);
 }
 
+__device__ __forceinline__ uint32_t upper_bits(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ uint32_t upper_bits(double v) { return (uint32_t)__double2hiint(v); }
+
 template <typename Real>
 struct RowSums {
     uint32_t* w;  // lo words, hi words (FP64: then the same of the remainders)
@@ -459,29 +475,86 @@ struct RowSums {
 #pragma unroll
         for (int k = 0; k < (int)(sizeof(Real) / 2); ++k) w[i + k * rows] = 0u;
     }
-    __device__ __forceinline__ void add(int32_t i, Real v, float unit) {
-        if constexpr (sizeof(Real) == 4) {
-            add_word(w + i, w + i + rows, (unsigned long long)__float2ll_rn(v * unit));
-        } else {
-            const double t = v * (double)unit;  // exact: the unit is a power of two
-            const double f = floor(t);
-            add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn(f));
-            add_word(w + i + 2 * rows, w + i + 3 * rows, (unsigned long long)__double2ll_rn((t - f) * 17592186044416.0));
-        }
+    __device__ __forceinline__ void add_units(int32_t i, double t) {  // t: in units, exact
+        const double f = floor(t);
+        add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn(f));
+        add_word(w + i + 2 * rows, w + i + 3 * rows, (unsigned long long)__double2ll_rn((t - f) * 17592186044416.0));
     }
-    __device__ __forceinline__ double get(int32_t i, float unit) const {
-        const double inv = 1.0 / (double)unit;
-        const long long q = (long long)((unsigned long long)w[i] | (unsigned long long)w[i + rows] << 32);
-        double r = (double)q * inv;
+    __device__ __forceinline__ void add(int32_t i, Real v) {
+        if constexpr (sizeof(Real) == 4) add_word(w + i, w + i + rows, (unsigned long long)__float2ll_rn(v * (float)kUnit));
+        else add_units(i, v * kUnit);
+    }
+    __device__ __forceinline__ void add_fine(int32_t i, Real v, double unit) {
+        if constexpr (sizeof(Real) == 4) add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn((double)v * unit));
+        else add_units(i, v * unit);
+    }
+    __device__ __forceinline__ unsigned long long units(int32_t i) const {
+        return (unsigned long long)w[i] | (unsigned long long)w[i + rows] << 32;
+    }
+    __device__ __forceinline__ double get(int32_t i, double unit = kUnit) const {
+        const double inv = 1.0 / unit;
+        double r = (double)(long long)units(i) * inv;
         if constexpr (sizeof(Real) == 8) {
             const unsigned long long p = (unsigned long long)w[i + 2 * rows] | (unsigned long long)w[i + 3 * rows] << 32;
             r += (double)p * (inv * (1.0 / 17592186044416.0));
         }
         return r;
     }
+    // After a refinement: the sum as a double instead.
+    __device__ __forceinline__ void set_double(int32_t i, double v) {
+        w[i] = (uint32_t)__double2loint(v);
+        w[i + rows] = (uint32_t)__double2hiint(v);
+    }
+    __device__ __forceinline__ double get_double(int32_t i) const {
+        return __hiloint2double((int)w[i + rows], (int)w[i]);
+    }
 };
 
+// Adds the rows of a row tile whose sums have too few units again, in units 2^36 times
+// finer at each level, until they have enough or no pair is left that is too small for the
+// level, and leaves every row's sum as a double.  What is added again stayed below
+// 2^kRowBits units of the level before, so nothing overflows.  `todo`: a bit per row that
+// still lacks units.  Called by the whole CTA, after a barrier, and ends with one.  Rare (see
+// above): it reads the row tile's pairs once more per level.
 template <typename Real>
+__device__ __noinline__ void refine_rows(RowSums<Real> R, uint32_t* todo, const GraphDev& G, int32_t tile) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int32_t nr = __ldg(G.row_tile + tile + 1) - __ldg(G.row_tile + tile);
+    const int32_t k0 = __ldg(G.row_step + tile), k1 = __ldg(G.row_step + tile + 1);
+    const Real* pairs = static_cast<const Real*>(G.pairs);
+    constexpr unsigned long long enough = 1ull << kRowBits<Real>;
+    double unit = kUnit;
+    bool more = true;
+    for (int level = 0;; ++level) {
+        for (int32_t i = tid; i < ((nr + 31) & ~31); i += kRowThreads) {  // whole warps: 32 rows, one word
+            const bool mine = i < nr && (level == 0 || (todo[i >> 5] >> (i & 31)) & 1u);
+            const bool again = mine && more && R.units(i) < enough;
+            const unsigned word = __ballot_sync(kFull, again);
+            if (again) R.clear(i);
+            else if (mine) R.set_double(i, R.get(i, unit));
+            if (lane == 0) todo[i >> 5] = word;
+        }
+        __syncthreads();
+        if (!more) return;
+        unit *= kFine;
+        const double least = (double)enough / unit;
+        bool small = false;  // a pair that the next level holds better
+        for (int32_t k = k0 + warp; k < k1; k += kRowWarps) {
+            const int2 st = __ldg(G.steps + k);
+            for (int32_t j = lane; j < st.y; j += 32) {
+                const int32_t i = __ldg(G.pair_row + st.x + j);
+                if (!((todo[i >> 5] >> (i & 31)) & 1u)) continue;
+                const Real v = __ldcg(pairs + st.x + j);
+                R.add_fine(i, v, unit);
+                small |= v != Real(0) && (double)v < least;
+            }
+        }
+        more = __syncthreads_or(small) && level + 1 < kFineLevels<Real>;
+    }
+}
+
+// kWatch: rows may get nothing but their sum (see refine_rows).
+template <typename Real, bool kWatch>
 __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParams P) {
     constexpr bool kFinal = std::is_same<Real, double>::value;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -489,6 +562,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
     __shared__ double part[kRowWarps][3];
     __shared__ unsigned long long words[6];          // fixed-point sums of the row tiles of `graph` finished here
     __shared__ int32_t s_idle, s_last, s_next;
+    __shared__ uint32_t todo[kWatch ? kMaxTileRows / 32 : 1];  // refine_rows
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     RowSums<Real> R{reinterpret_cast<uint32_t*>(smem_raw), P.max_rows};
     if (tid == 0) {
@@ -525,7 +599,12 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
         int32_t k = __ldg(G.row_step + rt.y) + warp;
         for (int32_t i = tid; i < nr; i += kRowThreads) R.clear(i);
         __syncthreads();  // the sums are clear, the view is set
-        const float unit = W.unit;
+        // Pairs below `tiny` are looked out for unless every row gets enough besides; positive
+        // floating-point numbers order like their (upper) bits, 0 wraps to the top.
+        constexpr double least = (double)(1ull << kRowBits<Real>) / kUnit;
+        [[maybe_unused]] const uint32_t tiny =
+            (W.personalised ? W.dmass : W.jump) >= kRowFloor<Real> ? 0u : upper_bits((Real)least) - 1u;
+        [[maybe_unused]] bool lost = false;
         const Real* pairs = static_cast<const Real*>(G.pairs) + lane;
         const uint16_t* prow = G.pair_row + lane;
         // a step's pairs are requested before the previous step's are added
@@ -549,7 +628,10 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
         auto add = [&](const Step& f) {
 #pragma unroll
             for (int j = 0; j < kStepPairs / 32; ++j)
-                if (32 * j < f.len) R.add((int32_t)f.row[j], f.v[j], unit);
+                if (32 * j < f.len) {
+                    R.add((int32_t)f.row[j], f.v[j]);
+                    if constexpr (kWatch) lost |= upper_bits(f.v[j]) - 1u < tiny;
+                }
         };
         Step fa, fb;
         load(fa);
@@ -559,7 +641,13 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
             load(fa);
             add(fb);
         }
-        __syncthreads();
+        [[maybe_unused]] bool refined = false;
+        if constexpr (kWatch) {
+            refined = __syncthreads_or(lost);
+            if (refined) refine_rows<Real>(R, todo, G, rt.y);
+        } else {
+            __syncthreads();
+        }
         double err = 0.0, dsum = 0.0, xsum = 0.0;
         // four rows of a thread at a time, their loads together
         for (int32_t i0 = tid; i0 < nr; i0 += 4 * kRowThreads) {
@@ -576,7 +664,10 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int32_t i = i0 + j * kRowThreads;
-                if (i < nr) finish_row<kFinal>(W, v0 + i, R.get(i, unit), xin[j], rd[j], err, dsum, xsum);
+                if (i < nr) {
+                    const double sum = kWatch && refined ? R.get_double(i) : R.get(i);
+                    finish_row<kFinal>(W, v0 + i, sum, xin[j], rd[j], err, dsum, xsum);
+                }
             }
         }
         err = warp_sum(err);
@@ -665,7 +756,6 @@ __global__ void k_init_states(GraphState* states, const GraphDev* graphs, const 
     s.max_iter = max_iter;
     s.done = 0;
     s.converged = 0;
-    s.fx_unit = alpha >= 0.0 && alpha <= 1.0 ? 4611686018427387904.f : 1099511627776.f;  // 2^62, 2^40
     s.personalised = personalised;
     states[gi] = s;
 }
@@ -733,8 +823,10 @@ int smem_optin() {
     cudaFuncSetAttribute(k_gather<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GatherSmem<float>));
     cudaFuncSetAttribute(k_gather<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GatherSmem<double>));
     constexpr int rows = kMaxTileRows * 2 * (int)sizeof(uint32_t);
-    cudaFuncSetAttribute(k_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
-    cudaFuncSetAttribute(k_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * rows);
+    cudaFuncSetAttribute(k_rows<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
+    cudaFuncSetAttribute(k_rows<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
+    cudaFuncSetAttribute(k_rows<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * rows);
+    cudaFuncSetAttribute(k_rows<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * rows);
     cudaGetLastError();
     cache[dev].store(optin, std::memory_order_release);
     return optin;
@@ -758,7 +850,7 @@ SweepParams make_params(Plan& plan, int use_cond) {
     P.acc = plan.d_acc.as<unsigned long long>();
     P.acc_sub = plan.nacc / std::max(1, plan.ngraphs);
     P.ctl = plan.d_ctl.as<Ctl>();
-    P.cond = plan.cond;
+    P.cond = 0;
     P.use_cond = use_cond;
     P.ngraphs = plan.ngraphs;
     smem_optin();
@@ -899,10 +991,10 @@ int plan_build(Plan& plan, egpr_graph* const* graphs, int32_t count, cudaStream_
 }
 
 // The sweeps as a CUDA graph: a while node whose body is the two phases.
-int plan_capture_loop(Plan& plan, cudaStream_t stream) {
-    (void)stream;
-    if (plan.cg_exec) return EGPR_SUCC;
-    if (plan.cg_failed) return EGPR_DEVICE_ERR;
+static int plan_capture_loop(Plan& plan, bool watch) {
+    Plan::Loop& L = plan.loops[watch];
+    if (L.exec) return EGPR_SUCC;
+    if (L.failed) return EGPR_DEVICE_ERR;
     cudaGraph_t cg = nullptr;
     cudaGraphExec_t ex = nullptr;
     cudaGraphConditionalHandle h = 0;
@@ -921,8 +1013,8 @@ int plan_capture_loop(Plan& plan, cudaStream_t stream) {
     cp.conditional.size = 1;
     e = cudaGraphAddNode(&cnode, cg, nullptr, 0, &cp);
     if (e != cudaSuccess) goto fail;
-    plan.cond = h;
     P = make_params(plan, 1);
+    P.cond = h;
     args[0] = &P;
     kp.func = (void*)k_gather<float>;
     kp.gridDim = dim3((unsigned)plan.grid);
@@ -931,7 +1023,7 @@ int plan_capture_loop(Plan& plan, cudaStream_t stream) {
     kp.kernelParams = args;
     e = cudaGraphAddKernelNode(&gnode, cp.conditional.phGraph_out[0], nullptr, 0, &kp);
     if (e != cudaSuccess) goto fail;
-    kp.func = (void*)k_rows<float>;
+    kp.func = watch ? (void*)k_rows<float, true> : (void*)k_rows<float, false>;
     kp.gridDim = dim3((unsigned)plan.row_grid);
     kp.blockDim = dim3(kRowThreads);
     kp.sharedMemBytes = (unsigned)row_smem(plan, false);
@@ -939,14 +1031,13 @@ int plan_capture_loop(Plan& plan, cudaStream_t stream) {
     if (e != cudaSuccess) goto fail;
     e = cudaGraphInstantiate(&ex, cg, 0);
     if (e != cudaSuccess) goto fail;
-    plan.cg = cg;
-    plan.cg_exec = ex;
+    L.graph = cg;
+    L.exec = ex;
     return EGPR_SUCC;
 fail:
     cudaGetLastError();
     if (cg) cudaGraphDestroy(cg);
-    plan.cond = 0;
-    plan.cg_failed = true;
+    L.failed = true;
     return EGPR_DEVICE_ERR;
 }
 
@@ -963,20 +1054,25 @@ int launch_init(Plan& plan, double alpha, int32_t max_iter, double tol, bool per
     return cuda_ok(cudaGetLastError(), "init launch");
 }
 
-int launch_loop(Plan& plan, int32_t max_iter, cudaStream_t stream, int32_t* launches) {
+bool rows_need_watch(const Plan& plan, double alpha, bool personalised) {
+    return personalised || !((1.0 - alpha) / (double)plan.max_n >= kRowFloor<float>);
+}
+
+int launch_loop(Plan& plan, int32_t max_iter, bool watch, cudaStream_t stream, int32_t* launches) {
     *launches = -1;  // counted on the device (Ctl::launches, sweeps)
-    if (graph_loop_enabled() && plan_capture_loop(plan, stream) == EGPR_SUCC)
-        return cuda_ok(cudaGraphLaunch(plan.cg_exec, stream), "graph launch");
+    if (graph_loop_enabled() && plan_capture_loop(plan, watch) == EGPR_SUCC)
+        return cuda_ok(cudaGraphLaunch(plan.loops[watch].exec, stream), "graph launch");
     // Plain launches; a sweep with no active graph returns at once.
     SweepParams P = make_params(plan, 0);
     for (int32_t it = 0; it < max_iter; ++it) {
         k_gather<float><<<plan.grid, 32 * kGatherWarps<float>, gather_smem(false), stream>>>(P);
-        k_rows<float><<<plan.row_grid, kRowThreads, row_smem(plan, false), stream>>>(P);
+        if (watch) k_rows<float, true><<<plan.row_grid, kRowThreads, row_smem(plan, false), stream>>>(P);
+        else k_rows<float, false><<<plan.row_grid, kRowThreads, row_smem(plan, false), stream>>>(P);
     }
     return cuda_ok(cudaGetLastError(), "sweep launch");
 }
 
-int launch_finish(Plan& plan, bool correction, cudaStream_t stream, int32_t* launches) {
+int launch_finish(Plan& plan, bool correction, bool watch, cudaStream_t stream, int32_t* launches) {
     dim3 grid((unsigned)vertex_grid(plan.max_n), (unsigned)plan.ngraphs);
     int32_t l = 0;
     if (correction) {
@@ -985,7 +1081,8 @@ int launch_finish(Plan& plan, bool correction, cudaStream_t stream, int32_t* lau
         // The loop's last CTA left the queue reset; the control block keeps the sweep count.
         SweepParams P = make_params(plan, 0);
         k_gather<double><<<plan.grid, 32 * kGatherWarps<double>, gather_smem(true), stream>>>(P);
-        k_rows<double><<<plan.row_grid, kRowThreads, row_smem(plan, true), stream>>>(P);
+        if (watch) k_rows<double, true><<<plan.row_grid, kRowThreads, row_smem(plan, true), stream>>>(P);
+        else k_rows<double, false><<<plan.row_grid, kRowThreads, row_smem(plan, true), stream>>>(P);
         l += 3;
     }
     k_normalize<<<grid, kThreads, 0, stream>>>(plan.d_graphs.as<GraphDev>(), plan.d_states.as<GraphState>(),
