@@ -306,25 +306,38 @@ static int read_states(Plan& plan, int32_t idx, cudaStream_t s, SolveOut* o) {
     return EGPR_SUCC;
 }
 
-// Enqueues a single-vector solve: the binned sweep (opt-in), the one-kernel solve of
-// a small graph, or the graph's plan.
+// Ranks sum to 1 and are not negative: a row's sum is at most alpha.  The sweep's row
+// sums rely on it (sweep.cu); the one-kernel solve adds floating-point numbers and
+// takes any alpha.
+static bool alpha_bounded(double alpha) { return alpha >= 0.0 && alpha <= 1.0; }
+
+// Enqueues a single-vector solve: the binned sweep (opt-in), the one-kernel solve of a
+// small graph or of an alpha outside [0, 1], or the graph's plan.
 static int enqueue_single(egpr_graph* g, double alpha, int32_t max_iter, double tol, bool personalised,
                           uint32_t flags, cudaStream_t s, int32_t* host_launches) {
     if (g->bins) return bins_enqueue(g, alpha, max_iter, tol, personalised, flags, s, host_launches);
-    if (!g->small_state.p) return enqueue_plan(g->plan, alpha, max_iter, tol, personalised, flags, s, host_launches);
+    g->last_one_kernel = g->one_kernel || !alpha_bounded(alpha);
+    if (!g->last_one_kernel) return enqueue_plan(g->plan, alpha, max_iter, tol, personalised, flags, s, host_launches);
+    float* z = g->z0.as<float>();
+    double* z64 = g->z64.as<double>();
+    int rc;
+    if (!g->one_kernel) {  // z0 and z64 hold ranked sources only: values by vertex in a buffer of their own, kept
+        if ((rc = g->small_state.grow_on(sizeof(SmallState), s)) || (rc = g->vertex_z.grow_on((size_t)g->n * sizeof(double), s)))
+            return rc;
+        z = g->vertex_z.as<float>();
+        z64 = g->vertex_z.as<double>();  // the correction sweep's values, over both z buffers
+    }
     const SmallGraph G{g->n, g->nnz, g->in_row.as<int32_t>(), g->in_col.as<int32_t>(),
                        g->weighted ? g->in_w.as<float>() : nullptr, g->outw.as<double>(),
                        personalised ? g->tele.as<float>() : nullptr};
-    float* z = g->z0.as<float>();
-    const SmallWork V{g->small_state.as<SmallState>(), {g->x0.as<float>(), g->x1.as<float>()}, {z, z + g->n},
-                      g->z64.as<double>()};
+    const SmallWork V{g->small_state.as<SmallState>(), {g->x0.as<float>(), g->x1.as<float>()}, {z, z + g->n}, z64};
     *host_launches = 2;
     return small_solve(G, V, alpha, tol, max_iter, (flags & EGPR_FLAG_NO_CORRECTION) == 0, g->out.as<double>(), s);
 }
 
 // The state of a graph's last single-vector solve.
 static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
-    if (!g->bins && g->small_state.p) {
+    if (!g->bins && g->last_one_kernel) {
         SmallState st;
         int rc;
         if ((rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state")) ||
@@ -530,7 +543,7 @@ static uint64_t bits_of(double x) {
 int64_t egpr_graph::device_bytes() const {
     int64_t b = 0;
     for (const egpr::DevBuf* d : {&in_row, &in_col, &in_w, &outw, &dangling01, &rank, &idx, &sw_w, &tile_bits, &tile_pair,
-                            &pair_row, &row_step, &steps, &row_tile, &pairs, &scale, &tele, &x0, &x1, &z0, &out, &z64, &small_state, &plan.d_units,
+                            &pair_row, &row_step, &steps, &row_tile, &pairs, &scale, &tele, &x0, &x1, &z0, &out, &z64, &small_state, &vertex_z, &plan.d_units,
                             &plan.d_cta_unit, &plan.d_row_tiles, &plan.d_graphs, &plan.d_states, &plan.d_ndang,
                             &plan.d_ctl, &plan.d_acc})
         b += (int64_t)d->bytes;
@@ -552,7 +565,7 @@ static void destroy_graph_object(egpr_graph* g) {
     g->plan.release();
     for (DevBuf* b : {&g->in_row, &g->in_col, &g->in_w, &g->outw, &g->dangling01, &g->rank, &g->idx, &g->sw_w,
                       &g->tile_bits, &g->tile_pair, &g->pair_row, &g->row_step, &g->steps, &g->row_tile, &g->pairs, &g->scale, &g->tele,
-                      &g->seed_ids, &g->small_state, &g->x0, &g->x1, &g->z0, &g->out, &g->z64})
+                      &g->seed_ids, &g->small_state, &g->vertex_z, &g->x0, &g->x1, &g->z0, &g->out, &g->z64})
         b->release();
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
@@ -829,6 +842,7 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
     if (g->tune_spmm_chunk == 0) g->tune_spmm_chunk = spmm_chunk_for(g->nnz);
     // by source rank, whole 16-byte units; by vertex in the one-kernel solve
     const bool small = small_wanted(n, g->nnz);
+    g->one_kernel = small ? 1 : 0;
     const size_t nz = (size_t)std::max<int64_t>(z_stride(g->nsrc), small ? n : 0);
     if ((rc = g->scale.alloc(2 * nf)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
         (rc = g->z0.alloc(2 * nz * sizeof(float))) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nz * sizeof(double))) ||
@@ -1117,6 +1131,21 @@ int egpr_pagerank_multi(int32_t count, egpr_graph* const* graphs, double alpha, 
         }
     }
     if (live.empty()) return EGPR_SUCC;
+    if (!alpha_bounded(alpha)) {  // not for the plan's row sums: the graphs one after another
+        double kernel_s = 0.0;
+        for (size_t i = 0; i < live.size(); ++i) {
+            egpr_stats st;
+            if ((rc = solve_single(live[i], alpha, max_iter, tol, nullptr, flags, outs[live_idx[i]], &st))) return rc;
+            kernel_s += st.kernel_seconds;
+            if (stats) stats[live_idx[i]] = st;
+        }
+        if (stats)  // the whole call's times for every graph, as from the plan
+            for (int32_t i : live_idx) {
+                stats[i].kernel_seconds = kernel_s;
+                stats[i].total_seconds = wall_seconds() - t0;
+            }
+        return EGPR_SUCC;
+    }
     std::shared_ptr<MultiPlan> mp;
     if ((rc = get_multi_plan(live.data(), (int32_t)live.size(), &mp))) return rc;
     cudaStream_t s = mp->stream;

@@ -314,7 +314,10 @@ struct egpr_graph {
     // solve workspace
     egpr::DevBuf scale, tele, x0, x1, z0, out, z64;
     egpr::DevBuf seed_ids;         // seed set of a single-vector PPR solve
-    egpr::DevBuf small_state;      // solves run as one kernel (small.cu) when this is allocated
+    int32_t one_kernel = 0;        // single-vector solves run as one kernel (small.cu)
+    int32_t last_one_kernel = 0;   // the last one did (also for an alpha that the sweep does not take)
+    egpr::DevBuf small_state;      // its state
+    egpr::DevBuf vertex_z;         // its carried values where z0 and z64 are by source rank
     egpr::Plan plan;               // single-graph plan
     egpr::SpmmWork* spmm = nullptr; // batched personalised PageRank workspace
     egpr::BinLayout* bins = nullptr; // binned single-graph sweep (null: the other paths serve single solves)

@@ -1,7 +1,7 @@
 // The whole solve of a small graph in one cooperative kernel: single-vector
 // PageRank / personalised PageRank on an inbound CSR (pagerank.py:75-139 restated as
-// a pull), for prepared graphs of few entries (api.cu) and for the
-// no-allocation entry (noalloc.cu).
+// a pull), for prepared graphs of few entries (api.cu), for the no-allocation entry
+// (noalloc.cu), and for an alpha outside [0, 1] on a graph of any size.
 //
 // Such a graph sweeps in a few microseconds, about what one launch costs, and its
 // vectors live in L2, so nothing is laid out for it: a few lanes per row gather the
@@ -149,9 +149,9 @@ __device__ __forceinline__ void na_finish(const SmallGraph& G, int32_t r, double
         A.err += fabs((double)xo - (double)xin[r]);
         xout[r] = xo;
         const double o = __ldg(G.outw + r);
-        const float sc = o <= 1e-15 ? -1.f : (float)(alpha / o);
-        zout[r] = sc >= 0.f ? xo * sc : 0.f;
-        if (sc < 0.f) A.dsum += (double)xo;
+        const bool dangling = o <= 1e-15;
+        zout[r] = dangling ? 0.f : xo * (float)(alpha / o);
+        if (dangling) A.dsum += (double)xo;
         A.xsum += (double)xo;
     }
 }
@@ -261,7 +261,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
            double* ranks) {
     SmallState* st = V.st;
     const int32_t n = G.n;
-    const int32_t tid = (int32_t)(blockIdx.x * kThreadsNa + threadIdx.x), nthreads = (int32_t)(gridDim.x * kThreadsNa);
+    const int64_t tid = (int64_t)blockIdx.x * kThreadsNa + threadIdx.x, nthreads = (int64_t)gridDim.x * kThreadsNa;
     const double c1 = G.tele ? 0.0 : (1.0 - alpha) / (double)n, tol_n = tol * (double)n;
     uint32_t barrier = 0;
     bool ok = true;
@@ -269,12 +269,12 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
     // pagerank.py:118); count of dangling vertices
     const float x0 = (float)(1.0 / (double)n);
     int32_t dang = 0;
-    for (int32_t v = tid; v < n; v += nthreads) {
+    for (int64_t v = tid; v < n; v += nthreads) {
         const double o = __ldg(G.outw + v);
-        const float sc = o <= 1e-15 ? -1.f : (float)(alpha / o);
+        const bool dangling = o <= 1e-15;
         V.x[0][v] = x0;
-        V.z[0][v] = sc >= 0.f ? x0 * sc : 0.f;
-        dang += sc < 0.f ? 1 : 0;
+        V.z[0][v] = dangling ? 0.f : x0 * (float)(alpha / o);
+        dang += dangling ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) dang += __shfl_down_sync(kFullNa, dang, o);
     if ((threadIdx.x & 31) == 0 && dang) atomicAdd(&st->ndang, dang);
@@ -309,7 +309,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
     if (ok && correction) {
         // the last sweep again in FP64, from x_{k-1}
         const float* xp = V.x[(iter - 1) & 1];
-        for (int32_t u = tid; u < n; u += nthreads) {
+        for (int64_t u = tid; u < n; u += nthreads) {
             const double o = __ldg(G.outw + u);
             V.z64[u] = o <= 1e-15 ? 0.0 : alpha * (double)xp[u] / o;
         }
@@ -324,7 +324,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
     if (ok) {  // final normalisation (pagerank.py:134-139)
         const float* xl = V.x[iter & 1];
         const double inv = xsum > 0.0 ? 1.0 / xsum : 0.0;
-        for (int32_t v = tid; v < n; v += nthreads) {
+        for (int64_t v = tid; v < n; v += nthreads) {
             const double val = correction ? __ldcg(ranks + v) : (double)xl[v];
             ranks[v] = xsum > 0.0 ? val * inv : 1.0 / (double)n;
         }

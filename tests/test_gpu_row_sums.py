@@ -64,3 +64,51 @@ def test_tiny_ranks_keep_their_relative_precision(correction, bulk):
     assert (np.abs(got[chain] / ref[chain] - 1.0) <= 4 * (hops + 1) * 2.0 ** -24).all()
     assert np.abs(got - ref).sum() <= 1e-6 and np.array_equal(got, again)
     pg.close()
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("alpha,sweeps", [(-0.5, 12), (1.0, 12), (1.3, 8)])
+def test_alpha_outside_the_unit_interval(alpha, sweeps, weighted):
+    """The entries accept any alpha; rows may be negative then."""
+    graphs = [_random(n, 9 * n, n, weighted) for n in (40013, 3001)]
+    pgs = [_native.PreparedGraph(*g) for g in graphs]
+    o = {"alpha": alpha, "max_iter": sweeps, "tol": 0.0}
+    refs = [oracle.pagerank_pull(*g, **o)[0] for g in graphs]
+    p = np.zeros(len(graphs[0][0]) - 1)
+    p[[0, 7]] = 0.5
+    pref = oracle.pagerank_pull(*graphs[0], teleport=p, **o)[0]
+
+    # four roundings per sweep, each 2^-24 of terms that sum to about 1, and later sweeps
+    # multiply them by at most |alpha| each
+    bound = 4 * 2.0 ** -24 * sum(abs(alpha) ** j for j in range(sweeps)) * 1.1
+
+    def check(got, ref):
+        assert np.abs(got - ref).sum() <= bound
+
+    for correction in (True, False):
+        for pg, ref in zip(pgs, refs):
+            check(pg.pagerank(correction=correction, **o)[0], ref)
+            pg.enqueue(correction=correction, **o)
+            got, st = pg.collect()
+            check(got, ref)
+            assert st["iterations"] == sweeps
+        outs, sts = _native.pagerank_multi(pgs, correction=correction, **o)
+        for got, ref, st in zip(outs, refs, sts):
+            check(got, ref)
+            assert st["iterations"] == sweeps
+        check(pgs[0].pagerank(personalization=p, correction=correction, **o)[0], pref)
+    for pg in pgs:
+        pg.close()
+
+
+def test_alpha_outside_the_unit_interval_on_a_large_graph():
+    """Small ranks: a row's value is about 2^-21 here, and keeps FP32's relative precision."""
+    n, sweeps = (1 << 21) + 5, 3
+    V, E, W = _random(n, 9 * n, 5)
+    pg = _native.PreparedGraph(V, E, W)
+    o = {"alpha": 1.01, "max_iter": sweeps, "tol": 0.0}
+    ref, _, _ = oracle.pagerank_pull(V, E, W, **o)
+    got, _ = pg.pagerank(correction=False, **o)
+    # four roundings per sweep, 2^-24 of a value at most
+    assert np.abs(got - ref).sum() <= 4 * sweeps * 2.0 ** -24
+    pg.close()
