@@ -844,7 +844,7 @@ int egpr_graph_create(const int32_t* V, const int32_t* E, const double* W, int32
     const bool small = small_wanted(n, g->nnz);
     g->one_kernel = small ? 1 : 0;
     const size_t nz = (size_t)std::max<int64_t>(z_stride(g->nsrc), small ? n : 0);
-    if ((rc = g->scale.alloc(2 * nf)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
+    if ((rc = g->scale.alloc(nd)) || (rc = g->tele.alloc(nf)) || (rc = g->x0.alloc(nf)) || (rc = g->x1.alloc(nf)) ||
         (rc = g->z0.alloc(2 * nz * sizeof(float))) || (rc = g->out.alloc(nd)) || (rc = g->z64.alloc(nz * sizeof(double))) ||
         (small && (rc = g->small_state.alloc(sizeof(SmallState))))) {
         destroy_graph_object(g);

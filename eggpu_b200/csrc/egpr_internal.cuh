@@ -79,7 +79,7 @@ struct GraphDev {
     void* pairs;                // per pair: its sum (FP32, or FP64 in the correction sweep)
     const double* outw;      // n, FP64 out-weight sums
     const int32_t* rank;     // n, rank of each source, -1 for a vertex without out-edges
-    const float2* rowd;      // n, what finishing a row needs: alpha/outw (FP32, -1 for dangling), rank (int32 bits)
+    const double* scale;     // n, alpha/outw, 0 for a dangling vertex
     const float* tele;       // n, personalisation (NULL = uniform)
     float* x[2];             // ranks, double-buffered
     float* z[2];             // by source rank: x * alpha/outw, the value each out-edge carries

@@ -150,7 +150,7 @@ __device__ __forceinline__ void na_finish(const SmallGraph& G, int32_t r, double
         xout[r] = xo;
         const double o = __ldg(G.outw + r);
         const bool dangling = o <= 1e-15;
-        zout[r] = dangling ? 0.f : xo * (float)(alpha / o);
+        zout[r] = dangling ? 0.f : (float)(val * (alpha / o));  // rounded once, as in sweep.cu
         if (dangling) A.dsum += (double)xo;
         A.xsum += (double)xo;
     }
@@ -273,7 +273,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
         const double o = __ldg(G.outw + v);
         const bool dangling = o <= 1e-15;
         V.x[0][v] = x0;
-        V.z[0][v] = dangling ? 0.f : x0 * (float)(alpha / o);
+        V.z[0][v] = dangling ? 0.f : (float)(alpha / o / (double)n);
         dang += dangling ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) dang += __shfl_down_sync(kFullNa, dang, o);

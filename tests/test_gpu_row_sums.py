@@ -5,7 +5,7 @@ significands) stated beside it."""
 import numpy as np
 import pytest
 
-from eggpu_b200 import _native
+from eggpu_b200 import _native, synth
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -111,4 +111,20 @@ def test_alpha_outside_the_unit_interval_on_a_large_graph():
     got, _ = pg.pagerank(correction=False, **o)
     # four roundings per sweep, 2^-24 of a value at most
     assert np.abs(got - ref).sum() <= 4 * sweeps * 2.0 ** -24
+    pg.close()
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("scale,small", [(16, "1000000000"), (18, "0")])
+def test_rounding_errors_average_out(monkeypatch, scale, small, seed):
+    """Carried values are rounded once, independently: 2^-25 / sqrt(3) = 1.7e-8 rms each, and
+    the rows that make up the norm average over a hundred and more sources: 2e-9, bound 4e-9.
+    An error shared by all sources of one out-degree would not average (1e-8 was seen)."""
+    monkeypatch.setenv("EGPR_SMALL_NNZ", small)  # the one-kernel solve, the sweep
+    g = synth.rmat(scale=scale, edgefactor=16, seed=seed)
+    o = {"alpha": 0.85, "max_iter": 20, "tol": 0.0}
+    pg = _native.PreparedGraph(g.V, g.E)
+    got, _ = pg.pagerank(**o)
+    ref, _, _ = oracle.pagerank_pull(g.V, g.E, None, **o)
+    assert np.linalg.norm(got - ref) <= 4e-9 * np.linalg.norm(ref)
     pg.close()
