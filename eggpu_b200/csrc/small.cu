@@ -32,7 +32,9 @@ namespace {
 constexpr int kThreadsNa = 1024;
 constexpr int kWarpsNa = kThreadsNa / 32;
 constexpr int32_t kWideRow = 128;   // entries: longer rows are summed by a warp,
-constexpr int32_t kHugeRow = 1024;  // and these by the whole CTA
+constexpr int32_t kHugeRow = 1024;  // and these by the whole CTA (longer ones only where rows are long on average)
+constexpr int64_t kCtaEntries = 2048;  // a CTA more per so many entries, while there are rows for its warps
+constexpr int32_t kCtaRows = 4;     // rows per CTA from which long ones are left to the warps
 constexpr unsigned long long kBarrierNs = 2000000000ull;  // bound of a barrier wait (2 s)
 constexpr unsigned kFullNa = 0xffffffffu;
 
@@ -158,14 +160,15 @@ __device__ __forceinline__ void na_finish(const SmallGraph& G, int32_t r, double
 
 // One sweep over this CTA's rows: L lanes per row; units of 32 / L rows are dealt to
 // the CTAs in turn.  Rows of more than kWideRow entries follow, a warp each, and
-// those of more than kHugeRow, one at a time by the whole CTA.
+// those of more than huge_row, one at a time by the whole CTA.
 template <bool kFinal, int L>
-__device__ NaSums na_rows(const SmallGraph& G, const typename std::conditional<kFinal, double, float>::type* z,
+__device__ NaSums na_rows(const SmallGraph& G, int32_t huge_row, const typename std::conditional<kFinal, double, float>::type* z,
                           double jump, double alpha, const float* xin, float* xout, float* zout, double* ranks) {
     using Real = typename std::conditional<kFinal, double, float>::type;
     __shared__ unsigned s_wide[kWarpsNa], s_huge[kWarpsNa];
     __shared__ Real s_part[kWarpsNa];
     constexpr int kRows = 32 / L;
+    const int32_t wide_row = L == 32 ? huge_row : kWideRow;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % L, grp = lane / L;
     const int64_t stride = (int64_t)gridDim.x * kWarpsNa;  // units of all CTAs together
     const int64_t units = ((int64_t)G.n + kRows - 1) / kRows;
@@ -174,7 +177,7 @@ __device__ NaSums na_rows(const SmallGraph& G, const typename std::conditional<k
         const int64_t r = u * kRows + grp;
         int64_t b = 0, e = 0;
         if (r < G.n) na_range(G, (int32_t)r, b, e);
-        const bool mine = r < G.n && e - b <= kWideRow;
+        const bool mine = r < G.n && e - b <= wide_row;
         Real acc = mine ? na_sum<Real>(G, z, b, e, sub, L) : Real(0);
 #pragma unroll
         for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(kFullNa, acc, o);
@@ -190,8 +193,8 @@ __device__ NaSums na_rows(const SmallGraph& G, const typename std::conditional<k
         const int64_t r = row_at(t0 + threadIdx.x);
         int64_t b = 0, e = 0;
         if (r < G.n) na_range(G, (int32_t)r, b, e);
-        const unsigned wide = __ballot_sync(kFullNa, e - b > kWideRow && e - b <= kHugeRow);
-        const unsigned huge = __ballot_sync(kFullNa, e - b > kHugeRow);
+        const unsigned wide = __ballot_sync(kFullNa, e - b > wide_row && e - b <= huge_row);
+        const unsigned huge = __ballot_sync(kFullNa, e - b > huge_row);
         if (lane == 0) {
             s_wide[warp] = wide;
             s_huge[warp] = huge;
@@ -258,7 +261,7 @@ __device__ void na_reduce(unsigned long long* acc, NaSums A) {
 template <int L>
 __global__ void __launch_bounds__(kThreadsNa, 1)
 k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter, int32_t correction,
-           double* ranks) {
+           int32_t huge_row, double* ranks) {
     SmallState* st = V.st;
     const int32_t n = G.n;
     const int64_t tid = (int64_t)blockIdx.x * kThreadsNa + threadIdx.x, nthreads = (int64_t)gridDim.x * kThreadsNa;
@@ -287,7 +290,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
     while (ok && !conv && iter < max_iter) {
         unsigned long long* acc = st->acc[iter % 3];
         const int par = iter & 1;
-        na_reduce(acc, na_rows<false, L>(G, V.z[par], c1 + dmass, alpha, V.x[par], V.x[par ^ 1], V.z[par ^ 1], nullptr));
+        na_reduce(acc, na_rows<false, L>(G, huge_row, V.z[par], c1 + dmass, alpha, V.x[par], V.x[par ^ 1], V.z[par ^ 1], nullptr));
         ok = na_barrier(st, ++barrier);
         unsigned long long w[6];
 #pragma unroll
@@ -316,7 +319,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
         ok = na_barrier(st, ++barrier);
         if (ok) {
             unsigned long long* acc = st->acc[iter % 3];
-            na_reduce(acc, na_rows<true, L>(G, V.z64, c1 + dmass_prev, alpha, xp, nullptr, nullptr, ranks));
+            na_reduce(acc, na_rows<true, L>(G, huge_row, V.z64, c1 + dmass_prev, alpha, xp, nullptr, nullptr, ranks));
             ok = na_barrier(st, ++barrier);
             xsum = na_fx_join(__ldcg(acc + 4), __ldcg(acc + 5));
         }
@@ -349,19 +352,30 @@ int small_solve(const SmallGraph& graph, const SmallWork& work, double alpha, do
     SmallGraph G = graph;
     SmallWork V = work;
     int32_t correction = with_correction ? 1 : 0;
-    // lanes per row by the mean degree; one CTA per SM at most, fewer where every warp
-    // would not get a unit of rows
+    // lanes per row by the mean degree; one CTA per SM at most, fewer where there are
+    // neither rows nor entries for all warps.  A warp per row: with 16 lanes, rows above
+    // kWideRow would take the second pass of na_rows, 5 us per sweep (8,192 vertices of
+    // degree 96 and 130, 20 sweeps: 0.40 and 0.49 ms with 16 lanes, 0.31 and 0.31 with 32;
+    // many rows hide it: 131,072 of degree 96, 1.52 and 1.64 ms)
     const int64_t degree = G.nnz / G.n;
-    const int lanes = degree <= 6 ? 4 : degree <= 20 ? 8 : 16;
-    const void* kernel = lanes == 4   ? (const void*)k_na_solve<4>
-                         : lanes == 8 ? (const void*)k_na_solve<8>
-                                      : (const void*)k_na_solve<16>;
-    const int64_t per_cta = (int64_t)kWarpsNa * (32 / lanes);
-    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)G.n + per_cta - 1) / per_cta, sweep_grid()));
+    const int lanes = degree <= 6 ? 4 : degree <= 20 ? 8 : degree <= (G.n <= 65536 ? 90 : 110) ? 16 : 32;
+    const void* kernel = lanes == 4    ? (const void*)k_na_solve<4>
+                         : lanes == 8  ? (const void*)k_na_solve<8>
+                         : lanes == 16 ? (const void*)k_na_solve<16>
+                                       : (const void*)k_na_solve<32>;
+    const int64_t units = ((int64_t)G.n + 32 / lanes - 1) / (32 / lanes);
+    const int64_t want = std::min(units, std::max((units + kWarpsNa - 1) / kWarpsNa, G.nnz / kCtaEntries));
+    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, sweep_grid()));
     // an odd number of CTAs: dealt by a power of two, the heavy rows of an R-MAT graph
     // (ids with few bits set) would all fall to the first CTAs
     if (grid > 1 && grid % 2 == 0) --grid;
-    void* args[] = {&G, &V, &alpha, &tol, &max_iter, &correction, &ranks};
+    // Where rows are long on average and every CTA has several, the warps take them up to
+    // four times the mean, one each; the whole CTA on one row after another leaves most
+    // warps waiting (2,048 vertices with 4 M entries, 20 sweeps: 2.87 ms, 0.45 so)
+    int32_t huge_row = kHugeRow;
+    if (G.n >= kCtaRows * std::min<int64_t>(want, sweep_grid()))
+        huge_row = (int32_t)std::max<int64_t>(kHugeRow, std::min<int64_t>(4 * degree, INT32_MAX));
+    void* args[] = {&G, &V, &alpha, &tol, &max_iter, &correction, &huge_row, &ranks};
     k_na_reset<<<1, 1, 0, s>>>(V.st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)grid), dim3(kThreadsNa), args, 0, s);

@@ -49,7 +49,11 @@ def _noalloc(pg, weighted, **o):
 @pytest.mark.parametrize("n,degree,row,weighted", [
     (1, 1, 1, False), (3, 2, 0, True), (33, 3, 127, True), (1000, 3, 128, False), (1000, 8, 129, True),
     (2049, 10, 1023, True), (2049, 10, 1024, False), (2050, 30, 1025, True), (4096, 30, 9000, True),
-    (16384, 12, 20000, False), (20011, 5, 3000, True)])
+    (16384, 12, 20000, False), (20011, 5, 3000, True),
+    # more than 96 entries per row: a warp per row; rows around four times the mean, from
+    # which the whole CTA takes over; and few rows, of which the CTA takes all above 1024
+    (40, 99, 0, False), (700, 400, 1200, True), (700, 400, 1201, False), (700, 400, 1900, True),
+    (5, 3000, 0, True), (9, 1024, 0, False)])
 def test_small_solve_at_row_length_edges(monkeypatch, n, degree, row, weighted, correction):
     monkeypatch.delenv("EGPR_SMALL_NNZ", raising=False)
     V, E, W = _graph(n, degree, row, weighted)
