@@ -72,6 +72,7 @@ __global__ void k_na_reset(SmallState* st) {
 // Grid barrier number `k` (1, 2, ...) of the kernel; false when it gave up waiting
 // (the kernel then ends and reports EGPR_TIMEOUT).  The fences order every
 // thread's accesses: thread 0's cover its CTA through the CTA barriers.
+// The count of arrivals wraps in solves of very many sweeps: compared by difference.
 __device__ bool na_barrier(SmallState* st, uint32_t k) {
     __shared__ int32_t s_ok;
     __syncthreads();
@@ -79,10 +80,10 @@ __device__ bool na_barrier(SmallState* st, uint32_t k) {
         __threadfence();
         atomicAdd(&st->arrived, 1u);
         const uint32_t want = k * gridDim.x;
-        bool ok = __ldcg(&st->arrived) >= want;
+        bool ok = (int32_t)(__ldcg(&st->arrived) - want) >= 0;
         if (!ok) {
             const unsigned long long t0 = na_global_ns();
-            while (!(ok = *reinterpret_cast<volatile uint32_t*>(&st->arrived) >= want) &&
+            while (!(ok = (int32_t)(*reinterpret_cast<volatile uint32_t*>(&st->arrived) - want) >= 0) &&
                    na_global_ns() - t0 < kBarrierNs) {
             }
         }
@@ -93,7 +94,6 @@ __device__ bool na_barrier(SmallState* st, uint32_t k) {
     __syncthreads();
     return s_ok != 0;
 }
-
 
 // Rows are clamped to [0, nnz] and sources to [0, n): no access outside the inputs.
 __device__ __forceinline__ void na_range(const SmallGraph& G, int32_t r, int64_t& b, int64_t& e) {
