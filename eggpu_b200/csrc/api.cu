@@ -354,6 +354,13 @@ static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
     return bins_read_state(g, s, &o->iterations, &o->converged, &o->residual, &o->launches, &o->error);
 }
 
+// The message of a single-vector solve that ended with an error.
+static int solve_error(const egpr_graph* g, int code) {
+    t_last_error = !g->bins && g->last_one_kernel ? "a barrier of the one-kernel solve ran out of time"
+                                                  : "the sweeps ended before every graph was done";
+    return code;
+}
+
 static void fill_stats(egpr_stats* stats, const egpr_graph* g, const SolveOut& o, double kernel_s,
                        double total_s, int32_t launches) {
     if (!stats) return;
@@ -445,10 +452,7 @@ static int solve_single(egpr_graph* g, double alpha, int32_t max_iter, double to
         return rc;
     SolveOut o;
     if ((rc = read_single_state(g, s, &o))) return rc;
-    if (o.error) {
-        t_last_error = "sweep launch cap reached";
-        return o.error;
-    }
+    if (o.error) return solve_error(g, o.error);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     fill_stats(stats, g, o, ms * 1e-3, wall_seconds() - t0, host_launches + o.launches);
@@ -1053,7 +1057,7 @@ int egpr_pagerank_collect(egpr_graph* g, double* out_ranks, egpr_stats* stats) {
         return rc;
     SolveOut o;
     if ((rc = read_single_state(g, s, &o))) return rc;
-    if (o.error) return o.error;
+    if (o.error) return solve_error(g, o.error);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     fill_stats(stats, g, o, ms * 1e-3, wall_seconds() - g->pending_t0, g->pending_launches + o.launches);

@@ -101,7 +101,10 @@ extern "C" EGPR_API int egpr_pagerank_device_noalloc(int32_t n, int64_t nnz, con
         SmallState h;
         if ((e = cudaMemcpy(&h, base, sizeof(egpr::SmallState), cudaMemcpyDeviceToHost)) != cudaSuccess)
             return set_cuda_error(e, "no-alloc solve state");
-        if (h.error) return h.error;
+        if (h.error) {
+            egpr::arg_error("egpr_pagerank_device_noalloc: a barrier of the solve ran out of time");
+            return h.error;
+        }
         const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         stats->iterations = h.iter;
         stats->converged = h.converged;

@@ -70,8 +70,8 @@ __global__ void k_na_reset(SmallState* st) {
 }
 
 // Grid barrier number `k` (1, 2, ...) of the kernel; false when it gave up waiting
-// (the kernel then ends and reports EGPR_TIMEOUT).  The fences order every
-// thread's accesses: thread 0's cover its CTA through the CTA barriers.
+// (the kernel then ends, reports EGPR_TIMEOUT and leaves NaN for ranks).  The fences
+// order every thread's accesses: thread 0's cover its CTA through the CTA barriers.
 // The count of arrivals wraps in solves of very many sweeps: compared by difference.
 __device__ bool na_barrier(SmallState* st, uint32_t k) {
     __shared__ int32_t s_ok;
@@ -324,13 +324,15 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
             xsum = na_fx_join(__ldcg(acc + 4), __ldcg(acc + 5));
         }
     }
-    if (ok) {  // final normalisation (pagerank.py:134-139)
+    if (ok && __ldcg(&st->error) == 0) {  // final normalisation (pagerank.py:134-139)
         const float* xl = V.x[iter & 1];
         const double inv = xsum > 0.0 ? 1.0 / xsum : 0.0;
         for (int64_t v = tid; v < n; v += nthreads) {
             const double val = correction ? __ldcg(ranks + v) : (double)xl[v];
             ranks[v] = xsum > 0.0 ? val * inv : 1.0 / (double)n;
         }
+    } else {  // a barrier ran out of time: no unfinished rank is taken for a result
+        for (int64_t v = tid; v < n; v += nthreads) ranks[v] = __longlong_as_double(0x7ff8000000000000ll);
     }
     if (threadIdx.x == 0) atomicMax(&st->t_end, na_global_ns());
 }

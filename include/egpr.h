@@ -301,8 +301,9 @@ EGPR_API int egpr_pagerank_csr(const int32_t* V, int32_t len_V, const int32_t* E
  * from the first to the last kernel of the solve, read from the GPU's global
  * timer; n <= 0 zeroes stats).  The whole solve is one cooperative kernel, which
  * ends at the stop rule: a sweep limit far above the sweeps needed costs
- * nothing, and the launch waits until its CTAs fit the device together.  The
- * array's device address is cached per device for the life of the process;
+ * nothing, and the launch waits until its CTAs fit the device together.  Its
+ * waits are bounded (2 s): one that runs out ends the solve with NaN ranks and,
+ * with stats, EGPR_TIMEOUT.  The array's device address is cached per device for the life of the process;
  * after cudaDeviceReset on that device the cached address is stale, so do not
  * reset a device between calls.
  */
