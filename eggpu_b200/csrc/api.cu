@@ -332,17 +332,29 @@ static int enqueue_single(egpr_graph* g, double alpha, int32_t max_iter, double 
                        personalised ? g->tele.as<float>() : nullptr};
     const SmallWork V{g->small_state.as<SmallState>(), {g->x0.as<float>(), g->x1.as<float>()}, {z, z + g->n}, z64};
     *host_launches = 2;
-    return small_solve(G, V, alpha, tol, max_iter, (flags & EGPR_FLAG_NO_CORRECTION) == 0, g->out.as<double>(), s);
+    std::atomic<int32_t>& in_flight = small_in_flight(g->device);
+    const int32_t others = in_flight.load(std::memory_order_relaxed) - g->counted;
+    if ((rc = small_solve(G, V, alpha, tol, max_iter, (flags & EGPR_FLAG_NO_CORRECTION) == 0, g->out.as<double>(), others, s)))
+        return rc;
+    if (!g->counted) in_flight.fetch_add(1, std::memory_order_relaxed);
+    g->counted = 1;
+    return EGPR_SUCC;
+}
+
+// The graph's one-kernel solve is done (or the graph goes).
+static void one_kernel_done(egpr_graph* g) {
+    if (g->counted) small_in_flight(g->device).fetch_sub(1, std::memory_order_relaxed);
+    g->counted = 0;
 }
 
 // The state of a graph's last single-vector solve.
 static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
     if (!g->bins && g->last_one_kernel) {
         SmallState st;
-        int rc;
-        if ((rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state")) ||
-            (rc = cuda_ok(cudaStreamSynchronize(s), "solve")))
-            return rc;
+        int rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state");
+        if (!rc) rc = cuda_ok(cudaStreamSynchronize(s), "solve");
+        one_kernel_done(g);
+        if (rc) return rc;
         o->iterations = st.iter;
         o->converged = st.converged;
         o->residual = st.residual;
@@ -563,6 +575,7 @@ static void destroy_graph_object(egpr_graph* g) {
     cudaGetDevice(&cur);
     if (g->device >= 0 && cur != g->device) cudaSetDevice(g->device);
     if (g->own_stream) cudaStreamSynchronize(g->own_stream);
+    one_kernel_done(g);
     spmm_work_release(g);
     delete g->bins;
     g->bins = nullptr;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -315,6 +316,7 @@ struct egpr_graph {
     egpr::DevBuf scale, tele, x0, x1, z0, out, z64;
     egpr::DevBuf seed_ids;         // seed set of a single-vector PPR solve
     int32_t one_kernel = 0;        // single-vector solves run as one kernel (small.cu)
+    int32_t counted = 0;           // a one-kernel solve of this graph is counted as in flight
     int32_t last_one_kernel = 0;   // the last one did (also for an alpha that the sweep does not take)
     egpr::DevBuf small_state;      // its state
     egpr::DevBuf vertex_z;         // its carried values where z0 and z64 are by source rank
@@ -389,8 +391,11 @@ int launch_finish(Plan& plan, bool correction, bool watch, cudaStream_t stream, 
 
 // The one-kernel solve (small.cu).
 bool small_wanted(int32_t n, int64_t nnz);  // prepared graphs it serves
+// others: one-kernel solves in flight on the device beside this one.
 int small_solve(const SmallGraph& graph, const SmallWork& work, double alpha, double tol, int32_t max_iter,
-                bool with_correction, double* ranks, cudaStream_t s);
+                bool with_correction, double* ranks, int32_t others, cudaStream_t s);
+// Number of one-kernel solves in flight on a device; the callers count theirs.
+std::atomic<int32_t>& small_in_flight(int device);
 
 // SpMM personalised PageRank (spmm.cu).  A batched sweep gathers a whole
 // 32-column panel per entry, about seven single-vector sweeps' worth, so

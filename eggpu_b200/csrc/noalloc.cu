@@ -95,7 +95,8 @@ extern "C" EGPR_API int egpr_pagerank_device_noalloc(int32_t n, int64_t nnz, con
     constexpr size_t N = kNoAllocMaxVertices;
     SmallWork V{reinterpret_cast<SmallState*>(base), {f, f + N}, {f + 2 * N, f + 3 * N},
                 reinterpret_cast<double*>(f + 2 * N)};  // the correction sweep's values, over both z buffers
-    if ((rc = small_solve(G, V, alpha, tol, max_iter, !(flags & EGPR_FLAG_NO_CORRECTION), ranks, s))) return rc;
+    const int32_t others = small_in_flight(dev).load(std::memory_order_relaxed);
+    if ((rc = small_solve(G, V, alpha, tol, max_iter, !(flags & EGPR_FLAG_NO_CORRECTION), ranks, others, s))) return rc;
     if (stats) {
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return set_cuda_error(e, "no-alloc solve");
         SmallState h;

@@ -34,12 +34,25 @@ constexpr int kWarpsNa = kThreadsNa / 32;
 constexpr int32_t kWideRow = 128;   // entries: longer rows are summed by a warp,
 constexpr int32_t kHugeRow = 1024;  // and these by the whole CTA (longer ones only where rows are long on average)
 constexpr int64_t kCtaEntries = 2048;  // a CTA more per so many entries, while there are rows for its warps
+constexpr int32_t kShares = 8;      // solves at a time that the SMs are shared by
 constexpr int32_t kCtaRows = 4;     // rows per CTA from which long ones are left to the warps
 constexpr unsigned long long kBarrierNs = 2000000000ull;  // bound of a barrier wait (2 s)
 constexpr unsigned kFullNa = 0xffffffffu;
 
-// Two's-complement fixed point in units of 2^-32 and 2^-64: integer adds, so
-// the totals do not depend on the order in which blocks finish.
+// Sums over rows that do not depend on how rows are dealt to threads: each number is
+// rounded to a multiple of a unit u so large that the sums stay exact in FP64 (adding and
+// subtracting 1.5 * 2^52 u rounds to one).  Ranks sum to 1: the FP32 sweeps' sums take
+// u = 2^-50, of which FP32 ranks of 2^-27 and more are multiples (all ranks of a uniform
+// teleport at the sizes served here), so nothing is lost there.  The FP64 sweep's rank
+// sum, by which the result is divided, has a second part for what that leaves, with u = 2^-64.
+__device__ __forceinline__ double na_round50(double v) { return (v + 6.0) - 6.0; }
+__device__ __forceinline__ double na_round64(double v) {
+    constexpr double m = 1.5 / 4096.0;
+    return (v + m) - m;
+}
+
+// Adds multiples of 2^-64 to two words, two's-complement fixed point in units of 2^-32 and
+// 2^-64: integer adds, so the totals do not depend on the order in which blocks finish.
 __device__ __forceinline__ void na_fx_add(unsigned long long* a, double v) {
     const double t = v * 4294967296.0;
     const double f = floor(t);
@@ -132,8 +145,10 @@ __device__ __forceinline__ Real na_sum(const SmallGraph& G, const Real* z, int64
     return acc;
 }
 
+// Sums over a CTA's rows.  FP32 sweep: residual, dangling mass, rank sum; FP64 sweep: the
+// rank sum's two parts.
 struct NaSums {
-    double err = 0.0, dsum = 0.0, xsum = 0.0;
+    double v[3] = {0.0, 0.0, 0.0};
 };
 
 // Finishes row r (see finish_row in sweep.cu).  jump: the dangling term, and the
@@ -143,18 +158,19 @@ __device__ __forceinline__ void na_finish(const SmallGraph& G, int32_t r, double
                                           const float* xin, float* xout, float* zout, double* ranks, NaSums& A) {
     const double val = G.tele ? (sum + (1.0 - alpha) * (double)__ldg(G.tele + r)) + jump : sum + jump;
     if (kFinal) {
-        A.err += fabs(val - (double)xin[r]);
         ranks[r] = val;
-        A.xsum += val;
+        const double t = na_round50(val);
+        A.v[0] += t;
+        A.v[1] += na_round64(val - t);
     } else {
         const float xo = (float)val;
-        A.err += fabs((double)xo - (double)xin[r]);
+        A.v[0] += na_round50(fabs((double)xo - (double)xin[r]));
         xout[r] = xo;
         const double o = __ldg(G.outw + r);
         const bool dangling = o <= 1e-15;
         zout[r] = dangling ? 0.f : (float)(val * (alpha / o));  // rounded once, as in sweep.cu
-        if (dangling) A.dsum += (double)xo;
-        A.xsum += (double)xo;
+        if (dangling) A.v[1] += na_round50((double)xo);
+        A.v[2] += na_round50((double)xo);
     }
 }
 
@@ -233,21 +249,17 @@ __device__ NaSums na_rows(const SmallGraph& G, int32_t huge_row, const typename 
     return A;
 }
 
-// Adds the CTA's sums to the accumulator words (fixed order inside the CTA).
+// Adds the CTA's sums to the accumulator words.
 __device__ void na_reduce(unsigned long long* acc, NaSums A) {
     __shared__ double red[kWarpsNa][3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        A.err += __shfl_xor_sync(kFullNa, A.err, o);
-        A.dsum += __shfl_xor_sync(kFullNa, A.dsum, o);
-        A.xsum += __shfl_xor_sync(kFullNa, A.xsum, o);
-    }
-    if (lane == 0) {
-        red[warp][0] = A.err;
-        red[warp][1] = A.dsum;
-        red[warp][2] = A.xsum;
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) A.v[i] += __shfl_xor_sync(kFullNa, A.v[i], o);
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) red[warp][i] = A.v[i];
     __syncthreads();
     if (threadIdx.x < 3) {
         double s = 0.0;
@@ -321,7 +333,7 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
             unsigned long long* acc = st->acc[iter % 3];
             na_reduce(acc, na_rows<true, L>(G, huge_row, V.z64, c1 + dmass_prev, alpha, xp, nullptr, nullptr, ranks));
             ok = na_barrier(st, ++barrier);
-            xsum = na_fx_join(__ldcg(acc + 4), __ldcg(acc + 5));
+            xsum = na_fx_join(__ldcg(acc), __ldcg(acc + 1)) + na_fx_join(__ldcg(acc + 2), __ldcg(acc + 3));
         }
     }
     if (ok && __ldcg(&st->error) == 0) {  // final normalisation (pagerank.py:134-139)
@@ -348,9 +360,14 @@ bool small_wanted(int32_t n, int64_t nnz) {
     return nnz <= most && n <= most;
 }
 
+std::atomic<int32_t>& small_in_flight(int device) {
+    static std::atomic<int32_t> count[64];
+    return count[device >= 0 && device < 64 ? device : 0];
+}
+
 // Sets the state up and enqueues the solve.
 int small_solve(const SmallGraph& graph, const SmallWork& work, double alpha, double tol, int32_t max_iter,
-                bool with_correction, double* ranks, cudaStream_t s) {
+                bool with_correction, double* ranks, int32_t others, cudaStream_t s) {
     SmallGraph G = graph;
     SmallWork V = work;
     int32_t correction = with_correction ? 1 : 0;
@@ -367,7 +384,13 @@ int small_solve(const SmallGraph& graph, const SmallWork& work, double alpha, do
                                        : (const void*)k_na_solve<32>;
     const int64_t units = ((int64_t)G.n + 32 / lanes - 1) / (32 / lanes);
     const int64_t want = std::min(units, std::max((units + kWarpsNa - 1) / kWarpsNa, G.nnz / kCtaEntries));
-    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, sweep_grid()));
+    // A solve alone takes all SMs; beside others it takes its share, so that they run at
+    // the same time (a cooperative launch waits until all its CTAs fit).  The results
+    // do not depend on the number of CTAs.  R-MAT scale 14, 20 sweeps, solves per second
+    // with 1, 4, 8 and 16 threads: 2,052, 7,277, 6,026 and 5,950; 2,051, 2,324, 2,332 and
+    // 2,306 where every solve takes all SMs
+    const int most = std::max(1, sweep_grid() / (1 + std::min(others, kShares - 1)));
+    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, most));
     // an odd number of CTAs: dealt by a power of two, the heavy rows of an R-MAT graph
     // (ids with few bits set) would all fall to the first CTAs
     if (grid > 1 && grid % 2 == 0) --grid;

@@ -78,6 +78,35 @@ def test_small_solve_at_row_length_edges(monkeypatch, n, degree, row, weighted, 
     pg.close()
 
 
+def test_solves_beside_others_give_the_same_bits(monkeypatch):
+    """A solve beside others takes fewer CTAs; its sums do not depend on their number."""
+    import threading
+
+    monkeypatch.delenv("EGPR_SMALL_NNZ", raising=False)
+    graphs = [_native.PreparedGraph(*_graph(n, d, row, w)) for n, d, row, w in
+              [(16384, 12, 3000, False), (9000, 20, 500, True), (1000, 8, 0, False), (2000, 90, 2500, True)] * 3]
+    o = {"max_iter": 30, "tol": 0.0}
+    alone = [pg.pagerank(**o)[0].copy() for pg in graphs]
+    wrong = []
+
+    def solve(i):
+        for _ in range(20):
+            if not np.array_equal(graphs[i].pagerank(**o)[0], alone[i]):
+                wrong.append(i)
+
+    threads = [threading.Thread(target=solve, args=(i,)) for i in range(len(graphs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for pg in graphs:  # all enqueued, then collected
+        pg.enqueue(**o)
+    for pg, want in zip(graphs, alone):
+        assert np.array_equal(pg.collect()[0], want)
+        pg.close()
+
+
 def test_noalloc_solve_can_be_captured():
     """The work is only enqueued (stats NULL), so a stream capture takes it; a replay
     solves again."""
