@@ -990,7 +990,7 @@ int egpr_graph_autotune(egpr_graph* g, uint32_t what, egpr_tuning* out) {
     if (g->nnz > 0 && (what & EGPR_TUNE_SPMM)) {
         double best = 1e30;
         int32_t bc = g->tune_spmm_chunk;
-        for (int32_t c : {512, 1024, 2048}) {
+        for (int32_t c : {128, 256, 512, 1024, 2048}) {  // spmm_chunk_for's values among them
             cudaStreamSynchronize(g->stream);
             spmm_work_release(g);
             g->tune_spmm_chunk = c;

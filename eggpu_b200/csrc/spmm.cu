@@ -951,8 +951,8 @@ int32_t default_spmm_chunk() {
 // and 16 ms.  With many panels a launch is long and the size matters little (256
 // columns on 16 M entries, 20 sweeps: 65.9, 61.7 and 62.4 ms with 256, 512 and 1024).
 int32_t spmm_chunk_for(int64_t entries) {
-    const int64_t want = entries / ((int64_t)8 * kSpWarps * 148);
-    return want >= 384 ? 512 : want >= 192 ? 512 : want >= 96 ? 256 : 128;
+    const int64_t want = entries / ((int64_t)8 * kSpWarps * sweep_grid());
+    return want >= 192 ? 512 : want >= 96 ? 256 : 128;
 }
 
 // Per-graph SpMM workspace: the layout (entry stream and chunks, built on the

@@ -25,8 +25,8 @@ def test_autotune_picks_a_candidate_and_keeps_results():
     before, st0 = pg.pagerank(alpha=0.85, max_iter=100, tol=1e-6)
     t = pg.autotune()
     assert t["chunks_per_warp"] in (4, 8, 16) and t["row_cost"] in (2, 4, 8)
-    assert t["spmm_chunk"] in (512, 1024, 2048)
-    assert t["configs_tried"] == 12 and t["sweep_ms"] > 0 and t["spmm_sweep_ms"] > 0
+    assert t["spmm_chunk"] in (128, 256, 512, 1024, 2048)
+    assert t["configs_tried"] == 14 and t["sweep_ms"] > 0 and t["spmm_sweep_ms"] > 0
     assert pg.tuning() == {k: t[k] for k in ("chunks_per_warp", "row_cost", "spmm_chunk")}
     after, st1 = pg.pagerank(alpha=0.85, max_iter=100, tol=1e-6)
     ref, it, _ = oracle.pagerank_pull(g.V, g.E, None, alpha=0.85, max_iter=100, tol=1e-6)
@@ -40,6 +40,27 @@ def test_autotune_picks_a_candidate_and_keeps_results():
                                           teleport=_seed_teleport(g.n, sets[j]))
         assert abs(sts[j]["iterations"] - it) <= 1
         assert np.abs(ranks[j] - ref).sum() <= L1_TOL
+
+
+@pytest.mark.parametrize("scale,default", [(14, 128), (18, 256), (20, 512)])
+def test_autotune_tries_the_default_tile(scale, default):
+    """The default follows the graph's size; the tuner keeps it or finds a faster one."""
+    g = synth.rmat(scale=scale, edgefactor=16, seed=47)
+    pg = _native.PreparedGraph(g.V, g.E)
+    assert pg.tuning()["spmm_chunk"] == default
+
+    def sweep_ms():
+        sets = synth.seed_sets(g.n, 32, 1, 1, seed=5)
+        def once(sweeps):  # noqa: E306
+            return min(pg.pagerank_seeds(sets, max_iter=sweeps, tol=0.0, correction=False)[1][0]["kernel_seconds"]
+                       for _ in range(3))
+        return (once(34) - once(2)) / 32 * 1e3
+
+    before = sweep_ms()
+    t = pg.autotune(sweep=False)
+    assert t["configs_tried"] == 5
+    assert sweep_ms() <= 1.1 * before  # a tenth for the timing's noise
+    pg.close()
 
 
 @pytest.mark.parametrize("cpw,rc,chunk", [(1, 0, 64), (64, 64, 4096), (3, 7, 96)])
@@ -65,7 +86,7 @@ def test_out_of_range_tuning_is_refused():
     for kw in ({"chunks_per_warp": 0}, {"row_cost": 65}, {"spmm_chunk": 100}, {"spmm_chunk": 32}):
         with pytest.raises(_native.EgprError):
             pg.set_tuning(**kw)
-    assert pg.tuning()["spmm_chunk"] in (512, 1024, 2048) or pg.tuning()["spmm_chunk"] % 32 == 0
+    assert pg.tuning()["spmm_chunk"] in (128, 256, 512)
 
 
 def test_autotune_choice_is_recorded_and_applied_to_new_graphs(tmp_path, monkeypatch):
