@@ -645,7 +645,9 @@ std::string tune_key(int dev, int32_t n, int64_t m, bool weighted) {
     }
     const int ln = floor_log2((uint64_t)std::max<int32_t>(n, 1));
     const int ld = floor_log2((uint64_t)std::max<int64_t>(m / std::max<int32_t>(n, 1), 1));
-    return name + "|n2^" + std::to_string(ln) + "|d2^" + std::to_string(ld) + "|w" + (weighted ? "1" : "0");
+    // l2: the two-phase sweep's layout; its parameters mean something else than those of
+    // the layout before, whose records (no such field) are not read
+    return name + "|l2|n2^" + std::to_string(ln) + "|d2^" + std::to_string(ld) + "|w" + (weighted ? "1" : "0");
 }
 
 bool tune_lookup(const std::string& key, egpr_tuning* out) {

@@ -107,6 +107,11 @@ def test_autotune_choice_is_recorded_and_applied_to_new_graphs(tmp_path, monkeyp
     h = synth.rmat(scale=14, edgefactor=16, seed=45)  # another graph of the same shape bucket
     ph = _native.PreparedGraph(h.V, h.E)
     assert ph.tuning() == {"chunks_per_warp": 16, "row_cost": 2, "spmm_chunk": 512}
+    # what a build with another layout recorded (no layout field in the key) is not read
+    assert "|l2|" in key
+    store.write_text(f"{key.replace('|l2|', '|')} 16 2 512 0.01\n")
+    assert _native.PreparedGraph(h.V, h.E).tuning() != {"chunks_per_warp": 16, "row_cost": 2, "spmm_chunk": 512}
+    store.write_text(f"{key} 16 2 512 0.01\n")
     ranks, st = ph.pagerank(alpha=0.85, max_iter=100, tol=1e-6)
     ref, it, _ = oracle.pagerank_pull(h.V, h.E, None, alpha=0.85, max_iter=100, tol=1e-6)
     assert abs(st["iterations"] - it) <= 1 and np.abs(ranks - ref).sum() <= L1_TOL
