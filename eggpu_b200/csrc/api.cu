@@ -966,7 +966,7 @@ int egpr_graph_autotune(egpr_graph* g, uint32_t what, egpr_tuning* out) {
     if ((rc = check_device(g))) return rc;
     egpr_tuning res;
     std::memset(&res, 0, sizeof(res));
-    if (g->nnz > 0 && (what & EGPR_TUNE_SWEEP)) {
+    if (g->nnz > 0 && (what & EGPR_TUNE_SWEEP) && !g->one_kernel) {  // that solve has no layout
         double best = 1e30;
         int32_t bc = g->tune_cpw, br = g->tune_rc;
         for (int32_t cpw : {4, 8, 16})
@@ -1014,7 +1014,7 @@ int egpr_graph_autotune(egpr_graph* g, uint32_t what, egpr_tuning* out) {
     res.chunks_per_warp = g->tune_cpw;
     res.row_cost = g->tune_rc;
     res.spmm_chunk = g->tune_spmm_chunk;
-    if (g->nnz > 0) tune_record(tune_key(g->device, g->n, g->m_input, g->weighted != 0), res);
+    if (res.configs_tried > 0) tune_record(tune_key(g->device, g->n, g->m_input, g->weighted != 0), res);
     if (out) *out = res;
     return EGPR_SUCC;
 }

@@ -159,7 +159,8 @@ typedef struct egpr_tuning {
  * Measures candidate layouts on this graph (a few fixed-count sweeps each,
  * timed on the device) and keeps the fastest: chunks_per_warp in {4, 8, 16}
  * x row_cost in {2, 4, 8} for the sweep, spmm_chunk in {128, 256, 512, 1024,
- * 2048} for the batched solve.  Results do not depend on the layout beyond FP32
+ * 2048} for the batched solve.  The sweep is left alone on a graph whose
+ * solves run as one kernel (up to 2^18 entries): that has no layout.  Results do not depend on the layout beyond FP32
  * rounding.  out (nullable) receives the chosen parameters and timings.
  * The choice is recorded per GPU model and graph-shape bucket (log2 of n,
  * log2 of the mean degree, weighted or not) in the file EGPR_TUNE_CACHE

@@ -13,6 +13,11 @@ pytestmark = pytest.mark.gpu
 L1_TOL = 1e-6
 
 
+@pytest.fixture(autouse=True)
+def _sweep_path(monkeypatch):
+    monkeypatch.setenv("EGPR_SMALL_NNZ", "0")  # these small graphs too take the sweep, whose layout is tuned
+
+
 def _seed_teleport(n, s):
     p = np.zeros(n)
     p[np.unique(s)] = 1.0
@@ -121,3 +126,17 @@ def test_autotune_choice_is_recorded_and_applied_to_new_graphs(tmp_path, monkeyp
                                                             "spmm_chunk": 512}
     monkeypatch.setenv("EGPR_TUNE_CACHE", "0")
     assert _native.PreparedGraph(h.V, h.E).tuning() != {"chunks_per_warp": 16, "row_cost": 2, "spmm_chunk": 512}
+
+
+def test_one_kernel_graphs_have_no_sweep_layout_to_tune(tmp_path, monkeypatch):
+    store = tmp_path / "tuning.txt"
+    monkeypatch.setenv("EGPR_TUNE_CACHE", str(store))
+    monkeypatch.delenv("EGPR_SMALL_NNZ")
+    g = synth.rmat(scale=12, edgefactor=16, seed=48)
+    pg = _native.PreparedGraph(g.V, g.E)
+    before = pg.tuning()
+    t = pg.autotune(sweep=True, spmm=False)
+    assert t["configs_tried"] == 0 and t["sweep_ms"] == 0 and pg.tuning() == before
+    assert not store.exists()  # nothing was measured, nothing is recorded
+    assert pg.autotune()["configs_tried"] == 5
+    pg.close()
