@@ -47,6 +47,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "batch_groups.h"
 #include "egpr_internal.cuh"
 
 namespace egpr {
@@ -1245,16 +1246,16 @@ int enqueue_group(egpr_graph* g, SpmmWork& w, double alpha, int32_t max_iter, do
 
 // Columns solved together.  A large graph's panels keep the GPU busy few at a time
 // (a panel sweep of 4 M entries takes about 0.1 ms), and a panel's results take as long
-// to copy out as many of its sweeps: there a group is three panels, whose results
-// travel while the next group is solved.  R-MAT scale 20, k = 256, 20 sweeps, 2.1 GB of
-// results: 104 ms in one group, 93.8, 83.4, 79.8 and 85.3 ms in groups of one to four
-// panels (fewer panels per launch fill the GPU less well, more leave more to copy at
-// the end).  Smaller graphs need many panels per launch and have little to copy.
-int32_t group_columns(const egpr_graph* g, const SpmmWork& w, int32_t k) {
+// to copy out as many of its sweeps: there the batch may be cut into groups (batch_groups.h).
+// Smaller graphs need many panels per launch and have little to copy.
+int32_t group_columns(const egpr_graph* g, const SpmmWork& w, int32_t k, int32_t sweeps) {
     constexpr int64_t kPanelEntries = 4 << 20;
-    constexpr int32_t kGroupPanels = 3;
     const bool large = w.epad >= kPanelEntries && (int64_t)g->n * kLanes * (int64_t)sizeof(double) >= (int64_t)16 << 20;
-    return std::min(k, (large ? kGroupPanels : kMaxPanels) * kLanes);
+    if (!large) return std::min(k, kMaxPanels * kLanes);
+    // two result buffers, the FP64 ranks and two FP32 iterates take 1,280 bytes per panel and
+    // vertex: up to 48 GB of them, but three panels in any case
+    const int32_t most = (int32_t)std::max<int64_t>(3, std::min<int64_t>(kMaxPanels, (int64_t)48e9 / ((int64_t)g->n * 1280)));
+    return std::min(k, batch_group_panels(w.epad, g->n, (k + kLanes - 1) / kLanes, sweeps, most) * kLanes);
 }
 
 }  // namespace
@@ -1309,7 +1310,7 @@ int ppr_batch_solve(egpr_graph* g, double alpha, int32_t max_iter, double tol, i
     if (!w.C && (rc = build_spmm_layout(g, w, s))) return rc;
     // Groups of columns: the results of a group are copied out (on a stream of their
     // own, from one of two buffers) while the next group is solved.
-    const int32_t group = group_columns(g, w, k), ngroups = (k + group - 1) / group;
+    const int32_t group = group_columns(g, w, k, expected_sweeps(alpha, tol, max_iter, n)), ngroups = (k + group - 1) / group;
     struct Events {
         std::vector<cudaEvent_t> ev;
         ~Events() {

@@ -16,7 +16,7 @@ def test_groups_of_columns_match_one_group(pinned, correction):
     g = synth.rmat(scale=16, edgefactor=80, seed=71)
     assert g.m + g.n >= 4 << 20 and g.n * 32 * 8 >= 16 << 20  # the sizes from which groups are used
     pg = _native.PreparedGraph(g.V, g.E)
-    sets = synth.seed_sets(g.n, 299, 1, 16, seed=9)  # groups of 96, 96, 96 and 11 columns
+    sets = synth.seed_sets(g.n, 299, 1, 16, seed=9)  # ten panels, the last one of 11 columns
     o = {"max_iter": 5, "tol": 0.0, "correction": correction}
     out = _native.pinned_empty((299, g.n)) if pinned else np.empty((299, g.n))
     got, st = pg.pagerank_seeds(sets, out=out, **o)
