@@ -105,8 +105,7 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, int64_t len, const uint32
 }
 
 // -------------------------------------------------------------- radix ------
-// LSD radix sort of (key, value) pairs with digits of kBits bits (8 in use):
-// a key of B bits takes ceil(B / kBits) passes.
+// LSD radix sort of (key, value) pairs with digits of kBits bits (8 to 10).
 template <int kBits>
 __global__ void __launch_bounds__(kThreads)
 k_radix_hist(const uint32_t* __restrict__ keys, int64_t len, int shift, int64_t ntiles,
@@ -129,95 +128,126 @@ k_radix_hist(const uint32_t* __restrict__ keys, int64_t len, int shift, int64_t 
 // lane order.  Global order = tile order (digit-major scanned histogram),
 // then warp order, then item order.  keys_out may be NULL (last pass: only
 // the values are needed).  kTwo: a second value array moves with the first.
+// The arrays go through one staging buffer in turn, and a value is loaded when its turn
+// comes, so four CTAs fit an SM (three with a buffer per array); every thread scans its
+// digits.  Preparation of R-MAT scale 25 weighted, page-locked input: 173 -> 159 ms with
+// the single 10-bit pass, scale 22 11.2 -> 10.2 ms.
+template <int kBits>
+struct RadixSmem {
+    static constexpr int kD = 1 << kBits;
+    uint32_t stage[kSortTile];    // the tile in digit order, one array at a time
+    uint32_t out[kD];             // where the digit's first item of the tile goes, minus its place in the tile
+    uint16_t hist[kWarps][kD];    // per warp: count of the digit, then the place of its first item in the tile
+    uint32_t warp_tot[kWarps];
+};
+
 template <int kBits, bool kTwo>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
 k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                 uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t len,
                 int shift, int64_t ntiles, const uint32_t* __restrict__ offsets,
                 const uint32_t* __restrict__ vals2_in, uint32_t* __restrict__ vals2_out) {
-    constexpr int kD = 1 << kBits;
-    extern __shared__ uint32_t radix_smem[];
-    uint32_t (*warp_hist)[kD] = reinterpret_cast<uint32_t (*)[kD]>(radix_smem);  // [kWarps][kD]
-    uint32_t* tile_off = radix_smem + kWarps * kD;                               // [kD]
+    constexpr int kD = 1 << kBits, kOwn = kD / kThreads;  // digits of a thread in the tile's scan
+    extern __shared__ __align__(16) unsigned char radix_smem[];
+    RadixSmem<kBits>& S = *reinterpret_cast<RadixSmem<kBits>*>(radix_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kWarps * kD; i += kThreads) radix_smem[i] = 0;
-    for (int d = tid; d < kD; d += kThreads) tile_off[d] = offsets[(int64_t)d * ntiles + blockIdx.x];
-    __syncthreads();
+    for (int i = tid; i < kWarps * kD / 2; i += kThreads) reinterpret_cast<uint32_t*>(&S.hist[0][0])[i] = 0u;
     const int64_t wbase = (int64_t)blockIdx.x * kSortTile + (int64_t)warp * 32 * kSortPerLane;
-    uint32_t key[kSortPerLane], val[kSortPerLane], val2[kTwo ? kSortPerLane : 1], rank[kSortPerLane];
+    uint32_t key[kSortPerLane], place[kSortPerLane];
+#pragma unroll
+    for (int r = 0; r < kSortPerLane; ++r) {
+        const int64_t idx = wbase + (int64_t)r * 32 + lane;
+        key[r] = idx < len ? keys_in[idx] : 0u;
+    }
+    __syncthreads();
     const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
     for (int r = 0; r < kSortPerLane; ++r) {
-        const int64_t idx = wbase + (int64_t)r * 32 + lane;
-        const bool valid = idx < len;
-        key[r] = valid ? keys_in[idx] : 0u;
-        val[r] = valid ? vals_in[idx] : 0u;
-        if (kTwo) val2[r] = valid ? vals2_in[idx] : 0u;
+        const bool valid = wbase + (int64_t)r * 32 + lane < len;
         const uint32_t d = (key[r] >> shift) & (kD - 1);
         const uint32_t tag = valid ? d : (uint32_t)(kD + lane);
         const uint32_t peers = __match_any_sync(0xffffffffu, tag);
-        const uint32_t before = valid ? warp_hist[warp][d] : 0u;
+        const uint32_t before = valid ? S.hist[warp][d] : 0u;
         __syncwarp();
-        if (valid && (peers & lt_mask) == 0u) warp_hist[warp][d] = before + __popc(peers);
+        if (valid && (peers & lt_mask) == 0u) S.hist[warp][d] = (uint16_t)(before + __popc(peers));
         __syncwarp();
-        rank[r] = before + __popc(peers & lt_mask);
+        place[r] = before + __popc(peers & lt_mask);
     }
     __syncthreads();
-    // per digit: the warps' prefix, and the tile's count (then its start in the tile)
-    uint32_t* dstart = tile_off + kD;  // [kD]
-    for (int d = tid; d < kD; d += kThreads) {
-        uint32_t run = 0;
+    // the tile's counts per digit, scanned: each thread a run of digits
+    uint32_t cnt[kOwn], run = 0;
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {
+        cnt[k] = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) cnt[k] += S.hist[w][tid * kOwn + k];
+        run += cnt[k];
+    }
+    uint32_t incl = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) S.warp_tot[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - run;  // of the thread's first digit
+    for (int w = 0; w < warp; ++w) at += S.warp_tot[w];
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {
+        const int d = tid * kOwn + k;
+        S.out[d] = offsets[(int64_t)d * ntiles + blockIdx.x] - at;
+        uint32_t p = at;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
-            uint32_t c = warp_hist[w][d];
-            warp_hist[w][d] = run;
-            run += c;
+            const uint32_t c = S.hist[w][d];
+            S.hist[w][d] = (uint16_t)p;
+            p += c;
         }
-        dstart[d] = run;
+        at += cnt[k];
     }
     __syncthreads();
-    if (warp == 0) {  // exclusive scan of the kD counts, one warp
-        uint32_t carry = 0;
-        for (int d0 = 0; d0 < kD; d0 += 32) {
-            const uint32_t c = dstart[d0 + lane];
-            uint32_t x = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            dstart[d0 + lane] = carry + x - c;
-            carry += __shfl_sync(0xffffffffu, x, 31);
-        }
-    }
-    __syncthreads();
-    // the tile in digit order in shared memory (same order as before: digit,
-    // then warp, then item), then each digit's run written out contiguously
-    uint32_t* skey = dstart + kD;          // [kSortTile]
-    uint32_t* sval = skey + kSortTile;     // [kSortTile]
-    uint32_t* sval2 = sval + kSortTile;    // [kSortTile] (kTwo)
 #pragma unroll
     for (int r = 0; r < kSortPerLane; ++r) {
-        const int64_t idx = wbase + (int64_t)r * 32 + lane;
-        if (idx < len) {
-            const uint32_t d = (key[r] >> shift) & (kD - 1);
-            const uint32_t lpos = dstart[d] + warp_hist[warp][d] + rank[r];
-            skey[lpos] = key[r];
-            sval[lpos] = val[r];
-            if (kTwo) sval2[lpos] = val2[r];
+        if (wbase + (int64_t)r * 32 + lane < len) {
+            place[r] += S.hist[warp][(key[r] >> shift) & (kD - 1)];
+            S.stage[place[r]] = key[r];
         }
     }
     __syncthreads();
+    // item i of the tile in digit order goes to dst: each digit's run is contiguous
     const int64_t tbase = (int64_t)blockIdx.x * kSortTile;
     const int nvalid = (int)(len - tbase < (int64_t)kSortTile ? len - tbase : (int64_t)kSortTile);
-    for (int i = tid; i < nvalid; i += kThreads) {
-        const uint32_t k = skey[i];
-        const uint32_t d = (k >> shift) & (kD - 1);
-        const uint32_t dst = tile_off[d] + ((uint32_t)i - dstart[d]);
-        if (keys_out) keys_out[dst] = k;
-        vals_out[dst] = sval[i];
-        if (kTwo) vals2_out[dst] = sval2[i];
+    uint32_t dst[kSortPerLane];
+#pragma unroll
+    for (int r = 0; r < kSortPerLane; ++r) {
+        const int i = tid + r * kThreads;
+        if (i < nvalid) {
+            const uint32_t k = S.stage[i];
+            dst[r] = S.out[(k >> shift) & (kD - 1)] + (uint32_t)i;
+            if (keys_out) keys_out[dst[r]] = k;
+        }
     }
+    auto move = [&](const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
+        uint32_t v[kSortPerLane];
+#pragma unroll
+        for (int r = 0; r < kSortPerLane; ++r) {
+            const int64_t idx = wbase + (int64_t)r * 32 + lane;
+            v[r] = idx < len ? in[idx] : 0u;
+        }
+        __syncthreads();  // the array before is read
+#pragma unroll
+        for (int r = 0; r < kSortPerLane; ++r)
+            if (wbase + (int64_t)r * 32 + lane < len) S.stage[place[r]] = v[r];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortPerLane; ++r) {
+            const int i = tid + r * kThreads;
+            if (i < nvalid) out[dst[r]] = S.stage[i];
+        }
+    };
+    move(vals_in, vals_out);
+    if (kTwo) move(vals2_in, vals2_out);
 }
 
 // -------------------------------------------------------------- graph ------
@@ -588,8 +618,7 @@ template <int kBits, bool kTwo>
 int radix_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t len, int shift,
                bool last, int64_t ntiles, uint32_t* hist, cudaStream_t s, const uint32_t* v2in, uint32_t* v2out) {
     constexpr int kD = 1 << kBits;
-    // warp histograms, tile offsets, digit starts, and the tile's keys and values
-    const size_t smem = ((size_t)(kWarps + 2) * kD + (kTwo ? 3 : 2) * (size_t)kSortTile) * sizeof(uint32_t);
+    const size_t smem = sizeof(RadixSmem<kBits>);
     // The shared-memory opt-in is a per-device attribute of the function: made
     // once per device (bit d of the mask; devices past 63 repeat it, which is
     // harmless).  Atomic: several host threads prepare graphs at once.
@@ -609,6 +638,13 @@ int radix_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_
     return EGPR_SUCC;
 }
 
+template <int kBits>
+int radix_pass_any(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t len, int shift,
+                   bool last, int64_t ntiles, uint32_t* hist, cudaStream_t s, const uint32_t* v2in, uint32_t* v2out) {
+    return v2in ? radix_pass<kBits, true>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out)
+                : radix_pass<kBits, false>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, nullptr, nullptr);
+}
+
 // Sorts (keys, vals) by `bits` bits of the keys from first_bit, stable.  After the
 // call the values are in the buffer *result_in_alt names; the keys are sorted
 // alongside except in the last pass, which writes values only.
@@ -619,31 +655,26 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_
     *result_in_alt = false;
     if (len <= 1 || bits <= 0) return EGPR_SUCC;
     int rc = EGPR_SUCC;
-    // 8-bit digits: with 4096-item tiles a digit's run averages 16 items, so
-    // the runs written out are 64-byte pieces (11-bit digits, one pass fewer,
-    // leave 2-item runs and were slower in total).  Where one or two 9-bit
-    // digits save a whole pass (25-bit keys: 9 + 8 + 8 instead of 8 + 8 + 8 + 1)
-    // they are used: 8-item runs, one pass of the data fewer.
+    // 8-bit digits: with 4096-item tiles a digit's run averages 16 items, so the
+    // runs written out are 64-byte pieces.  Where digits of 9 or 10 bits save a
+    // whole pass they are used (25-bit keys: 9 + 8 + 8 instead of 8 + 8 + 8 + 1; the
+    // sweep layout's sort by 628 blocks at R-MAT scale 25: one pass of 10).
     int passes = (bits + 7) / 8;
-    int nine = 0;  // leading passes of 9-bit digits
-    if (passes > 1 && bits <= 9 * (passes - 1)) {
-        passes -= 1;
-        nine = bits - 8 * passes;
-    }
+    while (passes > 1 && bits <= 10 * (passes - 1)) --passes;
     const int64_t ntiles = (len + kSortTile - 1) / kSortTile;
-    uint32_t* hist = tmp.get<uint32_t>((size_t)ntiles << (nine ? 9 : 8), &rc);
+    const int widest = std::max(8, (bits + passes - 1) / passes);
+    uint32_t* hist = tmp.get<uint32_t>((size_t)ntiles << widest, &rc);
     if (!hist) return rc;
     uint32_t *kin = keys, *vin = vals, *kout = keys_alt, *vout = vals_alt, *v2in = vals2, *v2out = vals2_alt;
     int shift = first_bit;
     for (int p = 0; p < passes; ++p) {
         const bool last = p == passes - 1 && !keys_needed;
-        if (p < nine)
-            rc = vals2 ? radix_pass<9, true>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out)
-                       : radix_pass<9, false>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, nullptr, nullptr);
-        else
-            rc = vals2 ? radix_pass<8, true>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out)
-                       : radix_pass<8, false>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, nullptr, nullptr);
-        shift += p < nine ? 9 : 8;
+        const int left = first_bit + bits - shift;  // the wider digits first
+        const int digit = std::max(8, (left + passes - p - 1) / (passes - p));
+        rc = digit == 10 ? radix_pass_any<10>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out)
+             : digit == 9 ? radix_pass_any<9>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out)
+                          : radix_pass_any<8>(kin, vin, kout, vout, len, shift, last, ntiles, hist, s, v2in, v2out);
+        shift += digit;
         if (rc) return rc;
         std::swap(kin, kout);
         std::swap(vin, vout);
