@@ -84,9 +84,17 @@ class GraphRegistry:
 
     @staticmethod
     def estimate_bytes(V, E, W):
+        """Device bytes that a prepared graph takes at most: the inbound CSR, the sweep's layout
+        (see GraphDev in egpr_internal.cuh) and the solve's vectors.  A graph without skew
+        has nearly a pair (10 bytes) per entry, an R-MAT graph 0.2."""
         n = len(V) - 1
         m = len(E)
-        return 4 * (n + 1) + 4 * m * (2 if W is not None else 1) + 8 * n + 4 * n + 24 * n + 16 * n + 64 * 1024
+        blocks = n // 22528 + 1
+        pairs = min(m, n * blocks) + m // 256  # at most one per entry, and per row and block, and one more per tile
+        steps = pairs // 128 + min(n // 256 + 1, 4096) * blocks
+        tiles = m // 256 + blocks
+        per_entry = 4 * (2 if W is not None else 1)
+        return (72 * n + per_entry * m + (256 * (per_entry - 2) + 68) * tiles + 10 * pairs + 8 * steps + 64 * 1024)
 
     def _prioritize(self, gid, pg):
         if pg.n > self.priority_max_n:

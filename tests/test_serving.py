@@ -297,6 +297,29 @@ def test_admission_by_bytes_evicts_idle_graphs(fake_engine):
     reg.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("kind,n,m", [("uniform", 1000, 8000), ("uniform", 100003, 1100000), ("uniform", 400000, 5000000),
+                                      ("rmat", 1 << 14, 16), ("rmat", 1 << 19, 16), ("ring", 70001, 70001)])
+def test_estimated_bytes_cover_the_prepared_graph(kind, n, m, weighted):
+    from eggpu_b200 import _native
+
+    rng = np.random.default_rng(n)
+    if kind == "rmat":
+        g = synth.rmat(scale=n.bit_length() - 1, edgefactor=m, seed=3, weighted=weighted)
+        V, E, W = g.V, g.E, g.W if weighted else None
+    else:
+        src = np.sort(rng.integers(0, n, m)) if kind == "uniform" else np.arange(n)
+        V = np.zeros(n + 1, np.int32)
+        V[1:] = np.cumsum(np.bincount(src, minlength=n))
+        E = rng.integers(0, n, m).astype(np.int32)
+        W = rng.random(m) if weighted else None
+    pg = _native.PreparedGraph(V, E, W)
+    need, estimate = pg.info()["device_bytes"], serving.GraphRegistry.estimate_bytes(V, E, W)
+    assert need <= estimate <= 2 * need
+    pg.close()
+
+
 def test_poisson_arrivals_are_seeded():
     a = serving.poisson_arrivals(1000.0, 500, seed=1)
     assert np.array_equal(a, serving.poisson_arrivals(1000.0, 500, seed=1))
