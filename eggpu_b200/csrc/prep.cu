@@ -713,7 +713,7 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t len, cudaStrea
 // Block and index of every inbound entry's source: (rank / kBlockSrc) in the high
 // bits, rank % kBlockSrc in the low kBlockBits (one-block layout: the rank).
 __global__ void k_source_codes(const int32_t* in_col, int64_t nnz, const int32_t* __restrict__ rank,
-                               int32_t blocked, uint32_t* code) {  // code may be in_col  // code may be in_col
+                               int32_t blocked, uint32_t* code) {  // code may be in_col
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
          i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t r = (uint32_t)rank[in_col[i]];

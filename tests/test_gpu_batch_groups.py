@@ -31,3 +31,24 @@ def test_groups_of_columns_match_one_group(pinned, correction):
     assert all(s["converged"] for s in st)
     assert np.abs(rule.sum(axis=1) - 1.0).max() < 1e-9
     pg.close()
+
+
+def test_groups_beside_an_open_session():
+    """A batch in groups leaves a session of the same graph alone, and the other way round."""
+    g = synth.rmat(scale=16, edgefactor=80, seed=72)
+    pg = _native.PreparedGraph(g.V, g.E)
+    sets = synth.seed_sets(g.n, 200, 1, 16, seed=10)
+    o = {"max_iter": 12, "tol": 0.0}
+    want, _ = pg.pagerank_seeds(sets, **o)
+    want = want.copy()
+    sess = _native.Session(pg, alpha=0.85, tol=0.0, slots=64)
+    slots = sess.admit(sets[:40], max_iter=12)
+    sess.step(5)
+    got, _ = pg.pagerank_seeds(sets, **o)  # while the session's columns are half way
+    assert np.array_equal(got, want)
+    done = list(sess.step(7))
+    assert sorted(done) == sorted(slots)
+    ranks, _ = sess.collect(slots)
+    assert np.abs(ranks - want[:40]).sum(axis=1).max() <= 1e-12
+    sess.close()
+    pg.close()

@@ -119,3 +119,45 @@ def test_every_cut_of_a_chunked_plan_gives_the_same_bits():
         assert all(np.array_equal(a, b) for a, b in zip(outs, first)), row_cost
     for pg in graphs:
         pg.close()
+
+
+@pytest.mark.parametrize("row_tiles", [1, 3, 64])
+def test_any_tuning_gives_the_same_ranks(layout, row_tiles):
+    """Row tiles of all sizes: other cuts of the rows change the order of no sum."""
+    rng = np.random.default_rng(8)
+    n = 60013
+    V, E, W = _csr(n, rng.integers(0, n, 700000), np.minimum(rng.zipf(1.3, 700000) - 1, n - 1), True, 9)
+    pg = _native.PreparedGraph(V, E, W)
+    o = {"max_iter": 5, "tol": 0.0}
+    ref, _, _ = oracle.pagerank_pull(V, E, W, alpha=0.85, **o)
+    pg.set_tuning(chunks_per_warp=row_tiles, row_cost=0 if row_tiles == 1 else row_tiles)
+    got, _ = pg.pagerank(**o)
+    assert np.abs(got - ref).sum() <= 1e-6
+    assert np.array_equal(got, pg.pagerank(**o)[0])
+    pg.close()
+
+
+@pytest.mark.parametrize("tol,max_iter", [(0.0, 7), (1e-9, 200)])
+def test_sweep_on_a_callers_stream(layout, tol, max_iter):
+    import torch
+
+    rng = np.random.default_rng(12)
+    n = 30011
+    V, E, W = _csr(n, rng.integers(0, n, 300000), rng.integers(0, n, 300000), True, 13)
+    pg = _native.PreparedGraph(V, E, W)
+    o = {"max_iter": max_iter, "tol": tol}
+    want, st = pg.pagerank(**o)
+    ref, it, _ = oracle.pagerank_pull(V, E, W, alpha=0.85, **o)
+    assert np.abs(want - ref).sum() <= 1e-6 and abs(st["iterations"] - it) <= 1
+    stream = torch.cuda.Stream()
+    pg.set_stream(stream.cuda_stream)
+    busy = torch.zeros(1 << 24, device="cuda")
+    with torch.cuda.stream(stream):
+        for _ in range(20):
+            busy.add_(1.0)  # the solve runs after the stream's earlier work
+    pg.enqueue(**o)
+    got, st2 = pg.collect()
+    assert np.array_equal(got, want) and st2["iterations"] == st["iterations"]
+    assert np.array_equal(pg.pagerank(**o)[0], want)
+    pg.set_stream(None)
+    pg.close()
