@@ -38,10 +38,10 @@
 // 2.01 ms per sweep, 0.97 of what 560 M sectors take at one per clock and SM, and
 // scale 22 took 0.222 ms.  Here k_gather is bound by issue and shared-memory
 // wavefronts (60% each of their peaks at scale 22: 90 us for 65 M entries, 11 M
-// pairs) and by HBM where there are weights (scale 25: 1.03 ms, 3.9 GB); k_rows is
-// bound by the latency of its loads (74 us and 0.70 ms).  Per sweep: scale 22 0.168
-// ms, scale 25 weighted 1.71 ms, Erdos-Renyi 1.5 M vertices 91 us (111 before), R-MAT
-// 100 K vertices 28 us (51 before).
+// pairs) and by HBM where there are weights (scale 25: 1.03 ms, 4.0 GB); k_rows is
+// bound by the latency of its loads (78 us and 0.70 ms, 1.7 GB).  Per sweep: scale 22 0.172
+// ms, scale 25 weighted 1.71 ms, Erdos-Renyi 1.5 M vertices 93 us (112 before), R-MAT
+// 100 K vertices 30 us (56 before).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -447,11 +447,13 @@ __global__ void __launch_bounds__(32 * kGatherWarps<Real>, 1) k_gather(SweepPara
 // A sum of at least 2^-36 (FP64: 2^-50) keeps 26 (56) bits, and so does every pair of that
 // size: less error than a chain of FP32 (FP64) adds has.  Smaller sums lose bits; they
 // matter only where a row gets nothing else, that is in a personalised solve on a
-// graph without dangling mass, far from the seeds.  There row tiles with smaller pairs
-// add their smallest rows again in finer units (refine_rows).
+// graph without dangling mass, far from the seeds.  There row tiles with small pairs
+// add their smallest rows again in finer units (refine_rows).  The looking out is in a
+// variant of the kernel for such solves: 50 personalised sweeps on 100 K vertices with
+// dangling ones 1.62 ms on the device instead of 1.59, on 1 M vertices without 4.01
+// instead of 3.83 (in every solve it would cost the plain ones 3%).
 constexpr double kUnit = 4611686018427387904.0;    // 2^62 units per 1
-constexpr int kFineShift = 36;                     // log2 between one unit and the next finer
-constexpr double kFine = 68719476736.0;            // 2^36
+constexpr double kFine = 68719476736.0;            // 2^36 between one unit and the next finer
 template <typename Real>
 constexpr int kRowBits = std::is_same<Real, double>::value ? 12 : 26;  // log2 of the units a sum has at least
 template <typename Real>
@@ -459,18 +461,20 @@ constexpr int kFineLevels = std::is_same<Real, double>::value ? 4 : 3;  // FP32:
 // A term of every row of at least this much makes the bits below the unit immaterial.
 template <typename Real>
 constexpr double kRowFloor = std::is_same<Real, double>::value ? 1.0 / 4503599627370496.0 : 1.0 / 274877906944.0;  // 2^-52, 2^-38
-__device__ __forceinline__ void add_word(uint32_t* lo, uint32_t* hi, unsigned long long q) {
+// Returns whether the upper word was left alone.
+__device__ __forceinline__ bool add_word(uint32_t* lo, uint32_t* hi, unsigned long long q) {
     const uint32_t ql = (uint32_t)q;
     uint32_t qh = (uint32_t)(q >> 32);
     if (ql) {
         const uint32_t old = atomicAdd(lo, ql);
         qh += old + ql < ql ? 1u : 0u;
     }
-    if (qh) atomicAdd(hi, qh);
+    if (qh) {
+        atomicAdd(hi, qh);
+        return false;
+    }
+    return true;
 }
-
-__device__ __forceinline__ uint32_t upper_bits(float v) { return __float_as_uint(v); }
-__device__ __forceinline__ uint32_t upper_bits(double v) { return (uint32_t)__double2hiint(v); }
 
 template <typename Real>
 struct RowSums {
@@ -480,14 +484,17 @@ struct RowSums {
 #pragma unroll
         for (int k = 0; k < (int)(sizeof(Real) / 2); ++k) w[i + k * rows] = 0u;
     }
-    __device__ __forceinline__ void add_units(int32_t i, double t) {  // t: in units, exact
+    __device__ __forceinline__ bool add_units(int32_t i, double t) {  // t: in units, exact
         const double f = floor(t);
-        add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn(f));
+        const bool low = add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn(f));
         add_word(w + i + 2 * rows, w + i + 3 * rows, (unsigned long long)__double2ll_rn((t - f) * 17592186044416.0));
+        return low;
     }
-    __device__ __forceinline__ void add(int32_t i, Real v) {
-        if constexpr (sizeof(Real) == 4) add_word(w + i, w + i + rows, (unsigned long long)__float2ll_rn(v * (float)kUnit));
-        else add_units(i, v * kUnit);
+    // Returns false for a pair of 2^-30 and more.
+    __device__ __forceinline__ bool add(int32_t i, Real v) {
+        if constexpr (sizeof(Real) == 4)
+            return add_word(w + i, w + i + rows, (unsigned long long)__float2ll_rn(v * (float)kUnit));
+        else return add_units(i, v * kUnit);
     }
     __device__ __forceinline__ void add_fine(int32_t i, Real v, double unit) {
         if constexpr (sizeof(Real) == 4) add_word(w + i, w + i + rows, (unsigned long long)__double2ll_rn((double)v * unit));
@@ -522,7 +529,7 @@ struct RowSums {
 // still lacks units.  Called by the whole CTA, after a barrier, and ends with one.  Rare (see
 // above): it reads the row tile's pairs once more per level.
 template <typename Real>
-__device__ __noinline__ void refine_rows(RowSums<Real> R, uint32_t* todo, const GraphDev& G, int32_t tile) {
+__device__ void refine_rows(RowSums<Real> R, uint32_t* todo, const GraphDev& G, int32_t tile) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int32_t nr = __ldg(G.row_tile + tile + 1) - __ldg(G.row_tile + tile);
     const int32_t k0 = __ldg(G.row_step + tile), k1 = __ldg(G.row_step + tile + 1);
@@ -531,6 +538,7 @@ __device__ __noinline__ void refine_rows(RowSums<Real> R, uint32_t* todo, const 
     double unit = kUnit;
     bool more = true;
     for (int level = 0;; ++level) {
+        bool any = false;
         for (int32_t i = tid; i < ((nr + 31) & ~31); i += kRowThreads) {  // whole warps: 32 rows, one word
             const bool mine = i < nr && (level == 0 || (todo[i >> 5] >> (i & 31)) & 1u);
             const bool again = mine && more && R.units(i) < enough;
@@ -538,9 +546,9 @@ __device__ __noinline__ void refine_rows(RowSums<Real> R, uint32_t* todo, const 
             if (again) R.clear(i);
             else if (mine) R.set_double(i, R.get(i, unit));
             if (lane == 0) todo[i >> 5] = word;
+            any |= again;
         }
-        __syncthreads();
-        if (!more) return;
+        if (!__syncthreads_or(any)) return;
         unit *= kFine;
         const double least = (double)enough / unit;
         bool small = false;  // a pair that the next level holds better
@@ -604,12 +612,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
         int32_t k = __ldg(G.row_step + rt.y) + warp;
         for (int32_t i = tid; i < nr; i += kRowThreads) R.clear(i);
         __syncthreads();  // the sums are clear, the view is set
-        // Pairs below `tiny` are looked out for unless every row gets enough besides; positive
-        // floating-point numbers order like their (upper) bits, 0 wraps to the top.
-        constexpr double least = (double)(1ull << kRowBits<Real>) / kUnit;
-        [[maybe_unused]] const uint32_t tiny =
-            (W.personalised ? W.dmass : W.jump) >= kRowFloor<Real> ? 0u : upper_bits((Real)least) - 1u;
-        [[maybe_unused]] bool lost = false;
+        [[maybe_unused]] uint32_t lost = 0u;  // 1: a small pair was added, 2: one that left no unit
         const Real* pairs = static_cast<const Real*>(G.pairs) + lane;
         const uint16_t* prow = G.pair_row + lane;
         // a step's pairs are requested before the previous step's are added
@@ -634,8 +637,8 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
 #pragma unroll
             for (int j = 0; j < kStepPairs / 32; ++j)
                 if (32 * j < f.len) {
-                    R.add((int32_t)f.row[j], f.v[j]);
-                    if constexpr (kWatch) lost |= upper_bits(f.v[j]) - 1u < tiny;
+                    const bool low = R.add((int32_t)f.row[j], f.v[j]);
+                    if (kWatch && low && f.v[j] != Real(0)) lost |= f.v[j] < Real(0.5 / kUnit) ? 3u : 1u;
                 }
         };
         Step fa, fb;
@@ -648,15 +651,23 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
         }
         [[maybe_unused]] bool refined = false;
         if constexpr (kWatch) {
-            refined = __syncthreads_or(lost);
-            if (refined) refine_rows<Real>(R, todo, G, rt.y);
+            // small sums matter unless every row gets enough besides
+            if ((W.personalised ? W.dmass : W.jump) >= kRowFloor<Real>) lost = 0u;
+            if (__syncthreads_or(lost != 0u)) {
+                const bool gone = __syncthreads_or(lost & 2u);  // else a sum of no units is 0
+                bool low = false;
+                for (int32_t i = tid; i < nr; i += kRowThreads)
+                    low |= R.units(i) < (1ull << kRowBits<Real>) && (gone || R.units(i) != 0ull);
+                refined = __syncthreads_or(low);
+                if (refined) refine_rows<Real>(R, todo, G, rt.y);
+            }
         } else {
             __syncthreads();
         }
         double err = 0.0, dsum = 0.0, xsum = 0.0;
-        // three rows of a thread at a time, their loads together (four need more registers than
-        // two CTAs per SM leave; two: 1% slower at scale 25)
-        constexpr int kRowsAhead = 3;
+        // three rows of a thread at a time, their loads together (four, or three with the watch,
+        // need more registers than two CTAs per SM leave; two: 1% slower at scale 25)
+        constexpr int kRowsAhead = kWatch ? 2 : 3;
         for (int32_t i0 = tid; i0 < nr; i0 += kRowsAhead * kRowThreads) {
             float xin[kRowsAhead];
             double scale[kRowsAhead];
