@@ -1,7 +1,7 @@
 // The binned single-graph sweep: one power-iteration sweep per launch over
 // the renumbered inbound CSR built by build_bin_layout (prep.cu).
 //
-// Per row v (a destination), as in the tile sweep (sweep.cu) and the
+// Per row v (a destination), as in the default sweep (sweep.cu) and the
 // reference's power iteration (easygraph/functions/centrality/pagerank.py:
 // 112-132) evaluated as a pull:
 //     x_new[v] = sum_{u -> v} w_uv * z[u] + jump,   z[u] = alpha * x[u] / outw[u]
@@ -669,10 +669,10 @@ int32_t lanes_for(int64_t len) {
 }  // namespace
 
 // The binned layout is built only on request (EGPR_BINS=1): measured on
-// B200 it runs 2.5-3x slower than the tile sweep (R-MAT scale 22: 0.64 against
-// 0.22 ms per sweep; scale 25 weighted: 6.6 against 2.6 ms), latency-bound on
+// B200 it runs 3.7-3.9x slower than the blocked sweep (R-MAT scale 22: 0.64 against
+// 0.17 ms per sweep; scale 25 weighted: 6.6 against 1.7 ms), latency-bound on
 // the dependent loads of each row group (row offsets, then sources, then
-// gathers), where the tile sweep loads a tile's sources one tile ahead.
+// gathers from global memory for all but the hub block's sources).
 bool bins_wanted(int32_t n, int64_t nnz) {
     const char* e = std::getenv("EGPR_BINS");
     return e && e[0] == '1' && n > 0 && nnz > 0;

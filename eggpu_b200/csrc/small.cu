@@ -14,9 +14,8 @@
 // sources, values, the row's data), about 5 us with its barrier on 1,000 vertices.
 // Measured per solve: 1,000 vertices, 6 sweeps: 51 us on the device (165 us as a
 // launch per phase); R-MAT scale 14, 5 sweeps: 141 us (160); the no-allocation entry on
-// 50,001 weighted vertices with a limit of 100 sweeps: 180 us (730 as a launch per
-// sweep).  On an R-MAT graph of 2.3 M entries a sweep takes 42 us, against 28 us in
-// the blocked sweep.
+// 50,001 weighted vertices with a limit of 100 sweeps: 176 us (720 as a launch per
+// sweep).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -351,9 +350,12 @@ k_na_solve(SmallGraph G, SmallWork V, double alpha, double tol, int32_t max_iter
 
 }  // namespace
 
-// Prepared graphs whose single-vector solves run here: up to 2^18 entries.  R-MAT with
-// 228 K entries: 141 us here, 160 us in the blocked sweep; with 2.3 M: 42 and 28 us per
-// sweep.  EGPR_SMALL_NNZ sets the limit (0: none).
+// Prepared graphs whose single-vector solves run here: up to 2^18 entries.  Whole calls
+// of 20 sweeps, here and in the blocked sweep: R-MAT with 111, 228, 468, 955 and 1,942 K
+// entries 410 and 554, 484 and 575, 539 and 596, 687 and 642, 846 and 724 us; uniform
+// with 131, 262, 524, 1,048 and 2,097 K entries 247 and 595, 311 and 584, 341 and 645,
+// 421 and 676, 549 and 810 us.  So the limit keeps to sizes where it wins on both
+// kinds.  EGPR_SMALL_NNZ sets it (0: none).
 bool small_wanted(int32_t n, int64_t nnz) {
     const char* e = std::getenv("EGPR_SMALL_NNZ");
     const int64_t most = e ? std::atoll(e) : (int64_t)1 << 18;

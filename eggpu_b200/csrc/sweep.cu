@@ -890,10 +890,13 @@ int64_t z_stride(int32_t nsrc) { return ((int64_t)nsrc + 31) & ~(int64_t)31; }
 
 int sweep_resident_warps() { return sweep_grid() * kGatherWarps<float>; }
 
-// CTAs for a persistent launch over `entries` inbound entries: one per
-// EGPR_CTA_ENTRIES entries (default 32768), at most `full`.  A small graph
-// then holds a few SMs instead of all of them, so solves of other graphs on
-// other streams run beside it (0: always the full grid).
+// CTAs of the sweep's first phase and of the batched solve over `entries` inbound
+// entries: one per EGPR_CTA_ENTRIES entries (default 32768), at most `full`.  A small
+// graph then holds a few SMs instead of all of them, so solves of other graphs on
+// other streams run beside it (0: always the full grid).  The second phase takes a CTA
+// per row tile, two per SM at most: its CTAs wait for nothing and leave after a few
+// microseconds.  Eight threads solving graphs of 0.8 M and 2 M entries: 6,083 and 3,619
+// solves/s, 4,798 and 2,497 with the single-phase sweep.
 int work_grid(int64_t entries, int full) {
     static const int64_t per = [] {
         const char* e = std::getenv("EGPR_CTA_ENTRIES");
