@@ -347,23 +347,27 @@ static void one_kernel_done(egpr_graph* g) {
     g->counted = 0;
 }
 
-// The state of a graph's last single-vector solve.
+// The state of a graph's last single-vector solve, after waiting for it.
 static int read_single_state(egpr_graph* g, cudaStream_t s, SolveOut* o) {
-    if (!g->bins && g->last_one_kernel) {
+    int rc;
+    if (g->bins) {
+        rc = bins_read_state(g, s, &o->iterations, &o->converged, &o->residual, &o->launches, &o->error);
+    } else if (g->last_one_kernel) {
         SmallState st;
-        int rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state");
+        rc = cuda_ok(cudaMemcpyAsync(&st, g->small_state.p, sizeof(st), cudaMemcpyDeviceToHost, s), "D2H state");
         if (!rc) rc = cuda_ok(cudaStreamSynchronize(s), "solve");
-        one_kernel_done(g);
-        if (rc) return rc;
-        o->iterations = st.iter;
-        o->converged = st.converged;
-        o->residual = st.residual;
-        o->launches = 0;
-        o->error = st.error;
-        return EGPR_SUCC;
+        if (!rc) {
+            o->iterations = st.iter;
+            o->converged = st.converged;
+            o->residual = st.residual;
+            o->launches = 0;
+            o->error = st.error;
+        }
+    } else {
+        rc = read_states(g->plan, 0, s, o);
     }
-    if (!g->bins) return read_states(g->plan, 0, s, o);
-    return bins_read_state(g, s, &o->iterations, &o->converged, &o->residual, &o->launches, &o->error);
+    one_kernel_done(g);  // also one that a later solve by another path followed
+    return rc;
 }
 
 // The message of a single-vector solve that ended with an error.

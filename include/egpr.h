@@ -181,7 +181,8 @@ EGPR_API int egpr_graph_set_tuning(egpr_graph* g, const egpr_tuning* in);
  * PageRank / personalised PageRank on a prepared graph.  personalization
  * (nullable, n values >= 0, not all zero) replaces the uniform teleport
  * vector after normalisation to sum 1; dangling mass stays uniform.
- * out_ranks[n] receives the normalised FP64 ranks.  stats may be NULL.
+ * out_ranks[n] receives the normalised FP64 ranks.  stats may be NULL.  alpha
+ * may lie outside [0, 1]; such solves run as one kernel on a graph of any size.
  */
 EGPR_API int egpr_pagerank(egpr_graph* g, double alpha, int32_t max_iter, double tol,
                   const double* personalization, uint32_t flags, double* out_ranks,

@@ -101,6 +101,21 @@ def test_alpha_outside_the_unit_interval(alpha, sweeps, weighted):
         pg.close()
 
 
+@pytest.mark.parametrize("first,second", [(1.2, 0.85), (0.85, 1.2)])
+def test_an_enqueued_solve_may_follow_one_of_the_other_path(first, second):
+    g = _random(40013, 9 * 40013, 40013)
+    pg = _native.PreparedGraph(*g)
+    o = {"max_iter": 6, "tol": 0.0}
+    pg.enqueue(alpha=first, **o)
+    pg.enqueue(alpha=second, **o)
+    got, st = pg.collect()
+    assert st["iterations"] == 6
+    assert np.array_equal(got, pg.pagerank(alpha=second, **o)[0])
+    ref, _, _ = oracle.pagerank_pull(*g, alpha=second, **o)
+    assert np.abs(got - ref).sum() <= 1e-6
+    pg.close()
+
+
 def test_alpha_outside_the_unit_interval_on_a_large_graph():
     """Small ranks: a row's value is about 2^-21 here, and keeps FP32's relative precision."""
     n, sweeps = (1 << 21) + 5, 3
