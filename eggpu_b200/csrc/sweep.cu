@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
             for (int j = 0; j < kStepPairs / 32; ++j)
                 if (32 * j < f.len) {
                     const bool low = R.add((int32_t)f.row[j], f.v[j]);
-                    if (kWatch && low && f.v[j] != Real(0)) lost |= f.v[j] < Real(0.5 / kUnit) ? 3u : 1u;
+                    if (kWatch && low && f.v[j] != Real(0)) lost |= f.v[j] < Real(1.0 / kUnit) ? 3u : 1u;
                 }
         };
         Step fa, fb;
