@@ -450,8 +450,8 @@ __global__ void __launch_bounds__(32 * kGatherWarps<Real>, 1) k_gather(SweepPara
 // graph without dangling mass, far from the seeds.  There row tiles with small pairs
 // add their smallest rows again in finer units (refine_rows).  The looking out is in a
 // variant of the kernel for such solves: 50 personalised sweeps on 100 K vertices with
-// dangling ones 1.62 ms on the device instead of 1.59, on 1 M vertices without 4.01
-// instead of 3.83 (in every solve it would cost the plain ones 3%).
+// dangling ones 1.59 ms on the device instead of 1.58, on 1 M vertices without 3.90
+// instead of 3.82 (in every solve it would cost the plain ones 3%).
 constexpr double kUnit = 4611686018427387904.0;    // 2^62 units per 1
 constexpr double kFine = 68719476736.0;            // 2^36 between one unit and the next finer
 template <typename Real>
@@ -665,9 +665,9 @@ __global__ void __launch_bounds__(kRowThreads, kRowTilesPerSm) k_rows(SweepParam
             __syncthreads();
         }
         double err = 0.0, dsum = 0.0, xsum = 0.0;
-        // three rows of a thread at a time, their loads together (four, or three with the watch,
-        // need more registers than two CTAs per SM leave; two: 1% slower at scale 25)
-        constexpr int kRowsAhead = kWatch ? 2 : 3;
+        // three rows of a thread at a time, their loads together (four, or two with the watch,
+        // need more registers than two CTAs per SM leave; two without: 1% slower at scale 25)
+        constexpr int kRowsAhead = kWatch ? 1 : 3;
         for (int32_t i0 = tid; i0 < nr; i0 += kRowsAhead * kRowThreads) {
             float xin[kRowsAhead];
             double scale[kRowsAhead];
